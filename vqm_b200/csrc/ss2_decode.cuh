@@ -12,7 +12,8 @@
 // holds exactly the per-sample values, so both paths round identically.
 // Integer YUV with a pure power-law transfer and at most 2x chroma
 // subsampling takes BlockLinearYuv (below), the same values with the
-// format's branches resolved; everything else BlockLinearGeneric.
+// format's branches resolved; linear, sRGB, ST 2084 and HLG images CurveRow;
+// everything else BlockLinearGeneric.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -524,6 +525,47 @@ __device__ __forceinline__ void ChromaFixed(const float* stage, int plane, int b
     }
 }
 
+// The bilinear chroma of the block at (x0, y0), both even, of tile (gx, gy),
+// from the staged window.
+__device__ __forceinline__ void ChromaFromStage(const DevSourceHead& s, const float* stage,
+                                                int plane, uint32_t gx, uint32_t gy, uint32_t x0,
+                                                uint32_t y0, float e[4][3]) {
+    if (s.chroma_pattern) {
+        const int bxs = static_cast<int>((x0 >> 1) - ((gx * kPrepTile) >> 1));
+        const int bys = static_cast<int>((y0 >> 1) - ((gy * kPrepTile) >> 1));
+        switch (s.chroma_pattern) {
+            case 1: ChromaFixed<0, 0>(stage, plane, bxs, bys, e); break;
+            case 2: ChromaFixed<1, 0>(stage, plane, bxs, bys, e); break;
+            case 3: ChromaFixed<0, 1>(stage, plane, bxs, bys, e); break;
+            default: ChromaFixed<1, 1>(stage, plane, bxs, bys, e); break;
+        }
+    } else {
+        const uint32_t sw = (kPrepTile >> s.sub_w) + 2;
+        // Window slot 0 of this block is chroma sample (cx - 1, cy - 1), the
+        // staged entry (cx - 1 - c0x, cy - 1 - c0y).
+        const int bxs = static_cast<int>((x0 >> s.sub_w) - ((gx * kPrepTile) >> s.sub_w));
+        const int bys = static_cast<int>((y0 >> s.sub_h) - ((gy * kPrepTile) >> s.sub_h));
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int xp = i & 1, yp = i >> 1;
+                const float* t =
+                    stage + p * plane + (bys + s.cslot[1][yp]) * static_cast<int>(sw) +
+                    bxs + s.cslot[0][xp];
+                const float* w = s.cweight[yp][xp];
+                // A first slot of 2 puts the second tap past the window: 0.
+                const bool xpast = s.cslot[0][xp] == 2, ypast = s.cslot[1][yp] == 2;
+                const float t0 = t[0], t1 = xpast ? 0.0f : t[1];
+                const float b0 = ypast ? 0.0f : t[sw];
+                const float b1 = xpast || ypast ? 0.0f : t[sw + 1];
+                e[i][1 + p] = __fmaf_rn(
+                    w[3], b1, __fmaf_rn(w[2], b0, __fmaf_rn(w[1], t1, __fmul_rn(w[0], t0))));
+            }
+        }
+    }
+}
+
 // BlockLinearGeneric for a yuv_fast image's block (bx, by) of the CTA's tile
 // (gx, gy) whose two columns and rows are inside the image: the same values,
 // with the format's branches resolved and the chroma taps read from the
@@ -573,39 +615,8 @@ __device__ __forceinline__ void BlockLinearYuv(const DevSourceHead& s, const flo
 #pragma unroll
         for (int i = 0; i < 4; ++i) e[i][0] = __fmaf_rn(v[i], s.scale[0], s.offset[0]);
     }
-    if (s.chroma_variant && s.chroma_pattern) {
-        const int bxs = static_cast<int>((x0 >> 1) - ((gx * kPrepTile) >> 1));
-        const int bys = static_cast<int>((y0 >> 1) - ((gy * kPrepTile) >> 1));
-        switch (s.chroma_pattern) {
-            case 1: ChromaFixed<0, 0>(stage, plane, bxs, bys, e); break;
-            case 2: ChromaFixed<1, 0>(stage, plane, bxs, bys, e); break;
-            case 3: ChromaFixed<0, 1>(stage, plane, bxs, bys, e); break;
-            default: ChromaFixed<1, 1>(stage, plane, bxs, bys, e); break;
-        }
-    } else if (s.chroma_variant) {
-        const uint32_t sw = (kPrepTile >> s.sub_w) + 2;
-        // Window slot 0 of this block is chroma sample (cx - 1, cy - 1), the
-        // staged entry (cx - 1 - c0x, cy - 1 - c0y).
-        const int bxs = static_cast<int>((x0 >> s.sub_w) - ((gx * kPrepTile) >> s.sub_w));
-        const int bys = static_cast<int>((y0 >> s.sub_h) - ((gy * kPrepTile) >> s.sub_h));
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int xp = i & 1, yp = i >> 1;
-                const float* t =
-                    stage + p * plane + (bys + s.cslot[1][yp]) * static_cast<int>(sw) +
-                    bxs + s.cslot[0][xp];
-                const float* w = s.cweight[yp][xp];
-                // A first slot of 2 puts the second tap past the window: 0.
-                const bool xpast = s.cslot[0][xp] == 2, ypast = s.cslot[1][yp] == 2;
-                const float t0 = t[0], t1 = xpast ? 0.0f : t[1];
-                const float b0 = ypast ? 0.0f : t[sw];
-                const float b1 = xpast || ypast ? 0.0f : t[sw + 1];
-                e[i][1 + p] = __fmaf_rn(
-                    w[3], b1, __fmaf_rn(w[2], b0, __fmaf_rn(w[1], t1, __fmul_rn(w[0], t0))));
-            }
-        }
+    if (s.chroma_variant) {
+        ChromaFromStage(s, stage, plane, gx, gy, x0, y0, e);
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -648,6 +659,270 @@ __device__ __forceinline__ void BlockLinearYuv(const DevSourceHead& s, const flo
             rgb[2 * h + 1][c] = q[h][c].y;
         }
     }
+}
+
+// The curve path (DevSource::curve): linear, sRGB, ST 2084 and HLG images.
+//
+// Its powers are ss2dm::pow and ss2dm::exp, value for value: the same
+// double-precision steps in the same order, for a normal finite float above 0,
+// with what surrounds them made cheaper. The mantissa and exponent go to
+// double by integer moves (a float's significand is a double's, shifted), the
+// floor by an addition rounded downwards, which leaves the integer in the
+// sum's low word, and 2^n by an addition to the exponent field; the table
+// entries of the logarithm come as one 16-byte shared-memory load. A row whose
+// values leave the direct range (float samples, codes far past the declared
+// depth) takes the shared functions.
+struct CurveTables {
+    double2 log[128];  // InvC, Log2InvC
+    double exp2[64];
+};
+__device__ __forceinline__ void StageCurveTables(CurveTables& t) {
+    for (uint32_t i = threadIdx.x; i < 128; i += blockDim.x)
+        t.log[i] = make_double2(ss2dm::InvC(static_cast<int>(i)),
+                                ss2dm::Log2InvC(static_cast<int>(i)));
+    for (uint32_t i = threadIdx.x; i < 64; i += blockDim.x)
+        t.exp2[i] = ss2dm::Exp2J(static_cast<int>(i));
+}
+// ss2dm::exp2d(t) rounded to float, for |t| < 1000.
+__device__ __forceinline__ float CurveExp2(double t, const CurveTables& tab) {
+    using ss2dm::K;
+    constexpr double kShift = 6755399441055744.0;  // 1.5 2^52
+    const double w = __dadd_rd(__fma_rn(t, 64.0, 0.5), kShift);
+    const int k = __double2loint(w);
+    const double f = __fma_rn(__dadd_rn(w, -kShift), -0.015625, t);
+    const double z = __dmul_rn(f, K(ss2dm::kLn2));
+    double p = K(ss2dm::kExpC6);
+    p = __fma_rn(p, z, K(ss2dm::kExpC5));
+    p = __fma_rn(p, z, K(ss2dm::kExpC4));
+    p = __fma_rn(p, z, K(ss2dm::kExpC3));
+    p = __fma_rn(p, z, K(ss2dm::kExpC2));
+    p = __fma_rn(p, z, K(ss2dm::kExpC1));
+    const double tj = tab.exp2[k & 63];
+    const double v = __fma_rn(tj, __dmul_rn(p, z), tj);  // in [0.5, 2]
+    return __double2float_rn(
+        __hiloint2double(__double2hiint(v) + ((k >> 6) << 20), __double2loint(v)));
+}
+// ss2dm::pow(x, y) for a normal finite x > 0 and |y| < 7.8.
+__device__ __forceinline__ float CurvePow(float x, float y, const CurveTables& tab) {
+    using ss2dm::K;
+    const uint32_t ix = __float_as_uint(x);
+    const double2 c = tab.log[(ix >> 16) & 127u];
+    const double m = __hiloint2double(static_cast<int>(0x3ff00000u | ((ix & 0x007fffffu) >> 3)),
+                                      static_cast<int>(ix << 29));
+    const double r = __fma_rn(m, c.x, -1.0);
+    double p = K(ss2dm::kLogC7);
+    p = __fma_rn(p, r, K(ss2dm::kLogC6));
+    p = __fma_rn(p, r, K(ss2dm::kLogC5));
+    p = __fma_rn(p, r, K(ss2dm::kLogC4));
+    p = __fma_rn(p, r, K(ss2dm::kLogC3));
+    p = __fma_rn(p, r, K(ss2dm::kLogC2));
+    const double ln1r = __fma_rn(__dmul_rn(r, r), p, r);
+    // The exponent as a double: 2^52 + its field, less 2^52 + 127 (exact).
+    const double e = __dadd_rn(__hiloint2double(0x43300000, static_cast<int>(ix >> 23)),
+                               -4503599627370623.0);
+    const double lg = __fma_rn(ln1r, K(ss2dm::kLog2E), __dadd_rn(c.y, e));
+    return CurveExp2(__dmul_rn(static_cast<double>(y), lg), tab);
+}
+
+// a / b for a divisor fixed at compile time: the product with the rounded
+// reciprocal, corrected once by the exact residual. For 1.055, 12.92,
+// 0.17883277 and 12 that is the correctly rounded quotient of every
+// significand of a (a test divides them all), and scaling by powers of two
+// changes nothing for a = 0 and 2^-100 <= |a| < 2^100.
+__device__ __forceinline__ float2 DivBy(float2 a, float b) {
+    const float r = 1.0f / b;
+    const float2 n = make_float2(-b, -b), rr = make_float2(r, r);
+    const float2 q = __fmul2_rn(a, rr);
+    return __ffma2_rn(__ffma2_rn(n, q, a), rr, q);
+}
+__device__ __forceinline__ float2 CurvePow2(float2 x, float y, const CurveTables& tab) {
+    return make_float2(CurvePow(x.x, y, tab), CurvePow(x.y, y, tab));
+}
+
+// TransferDecode's curves for two pixels whose values are 0 or at least 2^-100
+// and below 12 in magnitude (HLG's exponential overflows a float at 16.4).
+//
+// St2084Eotf. (Its scalar subtractions: a two-lane product feeding a two-lane
+// sum comes out as one fused operation.)
+__device__ __forceinline__ float2 CurveSt2084(float2 x, const CurveTables& tab) {
+    const bool la = x.x > 0.0f, lb = x.y > 0.0f;
+    const float2 xp = CurvePow2(make_float2(la ? x.x : 1.0f, lb ? x.y : 1.0f), 1.0f / 78.84375f,
+                                tab);
+    const float2 n = __fadd2_rn(xp, make_float2(-0.8359375f, -0.8359375f));
+    const float2 d = make_float2(__fsub_rn(18.8515625f, __fmul_rn(18.6875f, xp.x)),
+                                 __fsub_rn(18.8515625f, __fmul_rn(18.6875f, xp.y)));
+    const bool sa = la && n.x > 0.0f, sb = lb && n.y > 0.0f;
+    const float2 q = make_float2(sa ? __fdiv_rn(n.x, fmaxf(d.x, 1.17549435e-38f)) : 1.0f,
+                                 sb ? __fdiv_rn(n.y, fmaxf(d.y, 1.17549435e-38f)) : 1.0f);
+    const float2 w = CurvePow2(q, 1.0f / 0.1593017578125f, tab);
+    return make_float2(sa ? w.x : 0.0f, sb ? w.y : 0.0f);
+}
+// SrgbEotf.
+__device__ __forceinline__ float2 CurveSrgb(float2 x, const CurveTables& tab) {
+    const bool la = x.x <= 0.04045f, lb = x.y <= 0.04045f;
+    const float2 d = DivBy(__fadd2_rn(x, make_float2(0.055f, 0.055f)), 1.055f);
+    const float2 w =
+        CurvePow2(make_float2(la ? 1.0f : d.x, lb ? 1.0f : d.y), 2.4f, tab);
+    const float2 l = DivBy(x, 12.92f);
+    return make_float2(la ? l.x : w.x, lb ? l.y : w.y);
+}
+// AribInvOetf.
+__device__ __forceinline__ float2 CurveArib(float2 x, const CurveTables& tab) {
+    x = make_float2(fmaxf(x.x, 0.0f), fmaxf(x.y, 0.0f));
+    const float2 v = make_float2(fmaxf(x.x, 0.5f), fmaxf(x.y, 0.5f));
+    const float2 a =
+        DivBy(__fadd2_rn(v, make_float2(-0.55991073f, -0.55991073f)), 0.17883277f);
+    const double log2e = ss2dm::K(ss2dm::kLog2E);
+    const float2 e = make_float2(CurveExp2(__dmul_rn(static_cast<double>(a.x), log2e), tab),
+                                 CurveExp2(__dmul_rn(static_cast<double>(a.y), log2e), tab));
+    const float2 high = DivBy(__fadd2_rn(e, make_float2(0.28466892f, 0.28466892f)), 12.0f);
+    const float third = 1.0f / 3.0f;
+    const float2 low = __fmul2_rn(__fmul2_rn(x, x), make_float2(third, third));
+    return make_float2(x.x <= 0.5f ? low.x : high.x, x.y <= 0.5f ? low.y : high.y);
+}
+struct CurveValues {
+    float2 c[3];
+};
+// TransferRgb of two pixels by the shared functions.
+__device__ __noinline__ CurveValues RareRgb(const DevSourceHead& s, CurveValues v) {
+    float a[3] = {v.c[0].x, v.c[1].x, v.c[2].x}, b[3] = {v.c[0].y, v.c[1].y, v.c[2].y};
+    TransferRgb(s, a);
+    TransferRgb(s, b);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v.c[i] = make_float2(a[i], b[i]);
+    return v;
+}
+// TransferRgb of two pixels for the curve path's transfers.
+__device__ __forceinline__ void CurveRgb(const DevSourceHead& s, float2 (&c)[3],
+                                         const CurveTables& tab) {
+    if (s.transfer == 0) return;
+    {
+        bool direct = true;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            direct = direct && fabsf(c[i].x) < 12.0f && fabsf(c[i].y) < 12.0f;
+        if (s.curve == 1) {
+            const auto low = [](float v) { return v == 0.0f || fabsf(v) >= 7.8886091e-31f; };
+#pragma unroll
+            for (int i = 0; i < 3; ++i) direct = direct && low(c[i].x) && low(c[i].y);
+        }
+        if (!direct) {
+            const CurveValues v = RareRgb(s, CurveValues{{c[0], c[1], c[2]}});
+#pragma unroll
+            for (int i = 0; i < 3; ++i) c[i] = v.c[i];
+            return;
+        }
+    }
+    const float2 gain = make_float2(s.to_linear, s.to_linear);
+    if (s.transfer == 9) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = __fmul2_rn(gain, CurveSt2084(c[i], tab));
+    } else if (s.transfer == 4) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = CurveSrgb(c[i], tab);
+    } else if (s.transfer == 11) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = CurveArib(c[i], tab);
+        const float2 luma = __ffma2_rn(make_float2(s.kb, s.kb), c[2],
+                                       __ffma2_rn(make_float2(s.kg, s.kg), c[1],
+                                                  __fmul2_rn(make_float2(s.kr, s.kr), c[0])));
+        const float2 g = CurvePow2(make_float2(fmaxf(luma.x, 1.17549435e-38f),
+                                               fmaxf(luma.y, 1.17549435e-38f)),
+                                   0.2f, tab);
+        const float2 f = __fmul2_rn(g, gain);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = __fmul2_rn(c[i], f);
+    }
+}
+
+// The raw samples of four columns and two rows of the curve path's planes: as
+// the words of aligned loads (`words`: integer samples, the 4x2 block inside
+// the image), else read sample by sample when they are needed.
+struct CurveWords {
+    uint2 w[4][2];  // [plane][row]
+    bool words;     // every plane and row on a 4-byte boundary
+};
+__device__ __forceinline__ bool CurvePlane(const DevSourceHead& s, int p) {
+    return p == 0 || (p == 3 ? s.alpha != 0
+                             : s.family == 1 || (s.family == 2 && !s.chroma_variant));
+}
+__device__ __forceinline__ void LoadCurveWords(const DevSourceHead& s, bool aligned, uint32_t x,
+                                               uint32_t y, CurveWords& cw) {
+    cw.words = aligned && s.type <= 1 && x + 3 < s.width && y + 1 < s.height;
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) cw.w[p][h] = make_uint2(0, 0);
+    if (!cw.words) return;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        if (!CurvePlane(s, p)) continue;
+        const uint8_t* row =
+            s.plane[p] + static_cast<size_t>(y) * s.row_bytes[p] + (x << s.type);
+#pragma unroll
+        for (int h = 0; h < 2; ++h, row += s.row_bytes[p])
+            if (s.type == 0) cw.w[p][h].x = __ldg(reinterpret_cast<const uint32_t*>(row));
+            else cw.w[p][h] = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(row)),
+                                         __ldg(reinterpret_cast<const uint32_t*>(row + 4)));
+    }
+}
+// RawSample of columns x, x + 1 (x even, clamped to the image) of row y (row h
+// of the words, columns 2 hx on).
+__device__ __forceinline__ float2 CurveSamples(const DevSourceHead& s, const CurveWords& cw,
+                                               int p, uint32_t hx, uint32_t h, uint32_t x,
+                                               uint32_t y) {
+    float2 v;
+    if (cw.words) {
+        const uint2 w = h ? cw.w[p][1] : cw.w[p][0];
+        if (s.type == 0) {
+            const uint32_t b = hx ? w.x >> 16 : w.x;
+            v = make_float2(static_cast<float>(b & 0xffu), static_cast<float>((b >> 8) & 0xffu));
+        } else {
+            const uint32_t b = hx ? w.y : w.x;
+            v = make_float2(static_cast<float>(b & 0xffffu), static_cast<float>(b >> 16));
+        }
+        const int cls = p == 3 ? 2 : (p != 0 && s.family == 2 ? 1 : 0);
+        return __ffma2_rn(v, make_float2(s.scale[cls], s.scale[cls]),
+                          make_float2(s.offset[cls], s.offset[cls]));
+    }
+    y = min(y, s.height - 1);
+    return make_float2(RawSample(s, p, x, y), RawSample(s, p, min(x + 1, s.width - 1), y));
+}
+
+// BlockLinearGeneric's values for columns x, x + 1 of row y (row h of a 2x2
+// block) of a curve image, as two-lane channels; `cu` and `cv` are the pixels'
+// chroma where it is subsampled. Columns and rows past the image repeat its
+// last, as BlockLinearGeneric's clamped coordinates do.
+__device__ __forceinline__ void CurveRow(const DevSourceHead& s, const CurveWords& cw,
+                                         const CurveTables& tab, uint32_t hx, uint32_t h,
+                                         uint32_t x, uint32_t y, float2 cu, float2 cv,
+                                         float2 (&q)[3]) {
+    q[0] = q[1] = q[2] = CurveSamples(s, cw, 0, hx, h, x, y);
+    if (s.chroma_variant) {
+        q[1] = cu;
+        q[2] = cv;
+    } else if (s.family != 0) {
+        q[1] = CurveSamples(s, cw, 1, hx, h, x, y);
+        q[2] = CurveSamples(s, cw, 2, hx, h, x, y);
+    }
+    if (!s.identity1) ApplyMatrix2(s.m1, q);
+    if (s.alpha) {
+        const float2 a = CurveSamples(s, cw, 3, hx, h, x, y);
+        if (s.alpha == 2) {
+            const float ca = fminf(fmaxf(a.x, 0.0f), 1.0f), cb = fminf(fmaxf(a.y, 0.0f), 1.0f);
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                q[c] = make_float2(ca == 0.0f ? 0.0f : __fdiv_rn(q[c].x, ca),
+                                   cb == 0.0f ? 0.0f : __fdiv_rn(q[c].y, cb));
+        }
+        const float2 bg = make_float2(s.background, s.background);
+        const float2 target =
+            __fmul2_rn(__fadd2_rn(make_float2(1.0f, 1.0f), make_float2(-a.x, -a.y)), bg);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) q[c] = __ffma2_rn(a, q[c], target);
+    }
+    CurveRgb(s, q, tab);
+    if (!s.identity2) ApplyMatrix2(s.m2, q);
 }
 
 }  // namespace vqm_b200

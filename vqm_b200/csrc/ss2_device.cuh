@@ -88,7 +88,13 @@ struct DevSourceHead {
     // parity, so the host fixes the first window slot and the four tap
     // weights per parity. Also requires the YUV matrix to map every sample
     // code below the transfer power's fast-range limit.
+    // The curve path (BlockLinearCurve): any sample type and family, alpha
+    // included, whose transfer is linear, sRGB, ST 2084 or HLG, outside the
+    // constant-luminance mode; its subsampled chroma, if any, is integer,
+    // bilinear and by at most 2, with the phases below. 2: no value the
+    // transfer meets is tiny (CurveRgb); 1: it looks.
     uint8_t yuv_fast;
+    uint8_t curve;
     uint8_t chroma_pattern;    // 4:2:0 phases known at compile time: 1 + x type
                                // + 2 y type (type 0: siting offset 0, type 1:
                                // offset 1/4); 0: use cslot and cweight
@@ -139,17 +145,23 @@ struct DevPrepItem {
 
 // The prepare kernels, one per decode: 8-bit images by table (group 0),
 // yuv_fast images of even width and height (group 1: every 2x2 block is
-// whole, so its kernel carries no generic decode), every other image
-// (group 2).
-constexpr int kPrepGroups = 3;
+// whole, so its kernel carries no generic decode), curve images whose 2x2
+// blocks are whole where their chroma is subsampled (group 3), every other
+// image (group 2).
+constexpr int kPrepGroups = 4;
 inline int PrepGroup(const DevSource& s) {
     if (s.lut) return 0;
-    return s.yuv_fast && s.width % 2 == 0 && s.height % 2 == 0 ? 1 : 2;
+    const bool even = s.width % 2 == 0 && s.height % 2 == 0;
+    if (s.yuv_fast && even) return 1;
+    return s.curve && (even || !s.chroma_variant) ? 3 : 2;
 }
-// Whether an image fits the 4:2:0 chroma window of the 128-thread YUV
-// prepare kernel (4:2:0 chroma, or none subsampled).
-inline bool Yuv420Window(const DevSource& s) {
-    return !s.chroma_variant || (s.sub_w == 1 && s.sub_h == 1);
+// The launch's window flags (DevBatch::windows420) an image clears: its
+// group's bit, where the image does not fit the 4:2:0 chroma window of the
+// group's 128-thread kernel (4:2:0 chroma, or none subsampled).
+constexpr uint32_t kWindowsYuv = 1u, kWindowsCurve = 2u;
+inline uint32_t LargeWindow(const DevSource& s, int group) {
+    if (!s.chroma_variant || (s.sub_w == 1 && s.sub_h == 1)) return 0u;
+    return group == 1 ? kWindowsYuv : group == 3 ? kWindowsCurve : 0u;
 }
 
 struct DevBatch {
@@ -160,7 +172,7 @@ struct DevBatch {
     uint32_t blur_blocks;     // sum over segments of tiles
     const DevPair* pair;
     const DevSegment* seg;
-    const DevPrepItem* prep_item;  // group 0, then group 1, then group 2
+    const DevPrepItem* prep_item;  // group by group
     // Prefix tile offsets, each group's prep_items[g] + 1 entries in group
     // order.
     const uint32_t* prep_start;
@@ -172,8 +184,9 @@ struct DevBatch {
     uint32_t* blur_queue;        // the tile queue's next strip and exit count (0 between launches)
     uint32_t* status;            // nonzero: a kernel found bad input
     uint32_t half;               // 1: pyramid elements are binary16
-    uint32_t yuv420;             // 1: every image of the YUV prepare group
-                                 // has 4:2:0 chroma or none subsampled
+    uint32_t windows420;         // kWindowsYuv, kWindowsCurve: every image of
+                                 // that group has 4:2:0 chroma or none
+                                 // subsampled
     // The blur's 13 taps (offsets -6..6) as (w, w) pairs: the blur kernels
     // take them from the launch's parameter space, a constant bank like
     // __constant__ memory, so each batch carries its blur mode's filter.

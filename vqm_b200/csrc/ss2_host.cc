@@ -437,25 +437,11 @@ void HostBilinearPhase(uint32_t out_pos, float inv_scale, float shift, int centr
     w1 = t;
 }
 
-// DevSource's YUV fast-path fields: set when the format qualifies and every
-// block's bilinear phases are those of its parity (checked over block
-// indices across the whole coordinate range).
-// Sets the YUV fast path's constants (d.yuv_fast = 1 when it applies) and
-// returns a bound on the magnitude of the YUV matrix's outputs over every
-// sample code (infinity when the path does not apply).
-double FastYuvConstants(const vqm_cu_format& f, int mode, int tid, uint32_t chroma_filter,
-                        DevSource& d) {
-    const double none = HUGE_VAL;
-    d.yuv_fast = 0;
-    d.chroma_pattern = 0;
-    d.gamma = 0.0f;
-    std::memset(d.cslot, 0, sizeof(d.cslot));
-    std::memset(d.cweight, 0, sizeof(d.cweight));
-    if (!(f.family == 2 && f.type <= 1 && f.alpha == 0 && mode == 0 && tid >= 1 && tid <= 3 &&
-          f.subsample_w <= 1 && f.subsample_h <= 1 && (!d.chroma_variant || chroma_filter == 0)))
-        return none;
-    const float gammas[4] = {0.0f, 2.4f, 2.2f, 2.8f};  // TransferDecode cases 1-3
-    d.gamma = gammas[tid];
+// The bilinear chroma phases of an integer YUV format subsampled by at most
+// 2: each parity's window slot and tap weights (DevSource::cslot, cweight,
+// chroma_pattern), the same for every block (checked over block indices
+// across the whole coordinate range); false where they are not.
+bool ChromaPhases(const vqm_cu_format& f, DevSource& d) {
     float w[2][2][2];  // [axis][parity][tap]
     static const uint32_t kBlocks[] = {0, 1, 2, 3, 5, 77, 1000, 4095, 16383, 32767};
     for (int axis = 0; axis < 2; ++axis) {
@@ -477,12 +463,12 @@ double FastYuvConstants(const vqm_cu_format& f, int mode, int tid, uint32_t chro
                     w1_ref = w1;
                 } else if (s0 != s_ref || std::memcmp(&w0, &w0_ref, 4) ||
                            std::memcmp(&w1, &w1_ref, 4)) {
-                    return none;
+                    return false;
                 }
             }
             // Slot 2 (an axis that is not subsampled) puts the second tap past
             // the 3x3 window, where the generic decode reads 0.
-            if (s_ref < 0 || s_ref > 2) return none;
+            if (s_ref < 0 || s_ref > 2) return false;
             d.cslot[axis][par] = static_cast<int8_t>(s_ref);
             w[axis][par][0] = w0_ref;
             w[axis][par][1] = w1_ref;
@@ -492,7 +478,6 @@ double FastYuvConstants(const vqm_cu_format& f, int mode, int tid, uint32_t chro
     // device's ChromaFixed): offset 0 gives slots 0, 1 and weights
     // (1/4, 3/4), (3/4, 1/4); offset 1/4 gives slots 1, 1 and (1, 0),
     // (1/2, 1/2).
-    d.chroma_pattern = 0;
     if (f.subsample_w == 1 && f.subsample_h == 1) {
         int type[2] = {-1, -1};
         for (int axis = 0; axis < 2; ++axis) {
@@ -514,6 +499,40 @@ double FastYuvConstants(const vqm_cu_format& f, int mode, int tid, uint32_t chro
             d.cweight[yp][xp][2] = w[0][xp][0] * w[1][yp][1];
             d.cweight[yp][xp][3] = w[0][xp][1] * w[1][yp][1];
         }
+    return true;
+}
+
+// The decode paths with a chroma window of their own: sets yuv_fast and
+// gamma, curve, and the chroma phases both use. Returns a bound on the
+// magnitude of the YUV matrix's outputs over every sample code for the YUV
+// path (infinity when it does not apply).
+double FastDecodeConstants(const vqm_cu_format& f, int mode, int tid, uint32_t chroma_filter,
+                           DevSource& d) {
+    const double none = HUGE_VAL;
+    d.yuv_fast = 0;
+    d.curve = 0;
+    d.chroma_pattern = 0;
+    d.gamma = 0.0f;
+    std::memset(d.cslot, 0, sizeof(d.cslot));
+    std::memset(d.cweight, 0, sizeof(d.cweight));
+    const bool power = tid >= 1 && tid <= 3;
+    const bool curve = tid == 0 || tid == 4 || tid == 9 || tid == 11;
+    if (mode == 1 || !(power || curve)) return none;
+    const bool window = f.family == 2 && f.type <= 1 && f.subsample_w <= 1 &&
+                        f.subsample_h <= 1 && (!d.chroma_variant || chroma_filter == 0) &&
+                        ChromaPhases(f, d);
+    d.curve = curve && (window || !d.chroma_variant) ? 1 : 0;
+    // Integer samples' values are 0 or above 2^-100: a code times its scale
+    // plus the offset is a multiple of 2^-40, alpha is 0 or above 2^-17, and
+    // the matrix entries are 0 or above 2^-58 (0 can come out of the inversion
+    // as about 2^-55).
+    const float bg = std::fabs(d.background);
+    if (d.curve && f.type <= 1 &&
+        (f.alpha == 0 || (f.alpha == 1 && (bg == 0.0f || (bg >= 1e-6f && bg <= 4.0f)))))
+        d.curve = 2;
+    if (!(power && window && f.alpha == 0 && mode == 0)) return none;
+    const float gammas[4] = {0.0f, 2.4f, 2.2f, 2.8f};  // TransferDecode cases 1-3
+    d.gamma = gammas[tid];
     // The device's two-lane power takes every input from 2^-30 up without a
     // range check: every sample code the container can hold (whatever the
     // declared depth) must keep the YUV matrix's outputs below the power's
@@ -619,7 +638,7 @@ void BuildSourceConstants(const vqm_cu_format& f, uint32_t chroma_filter, float 
         d.cl[3] = static_cast<float>(1.0 - Rec709Oetf(kr));
     }
     d.background = background;
-    const double yuv_bound = FastYuvConstants(f, mode, tid, chroma_filter, d);
+    const double yuv_bound = FastDecodeConstants(f, mode, tid, chroma_filter, d);
     // 8-bit grey/RGB without alpha: every sample decodes independently of its
     // neighbours, so one table per image holds the whole transfer decode.
     d.lut = (f.type == 0 && (f.family == 0 || f.family == 1) && f.alpha == 0 && mode == 0 &&

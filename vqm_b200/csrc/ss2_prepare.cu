@@ -10,11 +10,12 @@
 // averaged, each level with a barrier among the threads it still needs.
 // Because the 2x2 box nests exactly, no CTA ever needs a neighbour's samples.
 //
-// Two kernels: 8-bit grey/RGB without alpha decode through the image's
+// Four kernels: 8-bit grey/RGB without alpha decode through the image's
 // 256-entry table in shared memory, reading four samples of a row with one
-// 32-bit load where the planes allow it; every other format runs the decode
-// of ss2_decode.cuh, whose YUV fast path (integer YUV, power-law transfer)
-// stages the tile's chroma window in shared memory first. Images whose
+// 32-bit load where the planes allow it; the YUV path (integer YUV, power-law
+// transfer) and the curve path (linear, sRGB, ST 2084 and HLG) of
+// ss2_decode.cuh stage the tile's chroma window in shared memory first; every
+// other format runs its generic decode. Images whose
 // linear samples the host has proved non-negative run a body whose cube
 // roots skip their range check (the same values). The XYB transform of two
 // pixels runs on Blackwell's two-lane FP32 instructions, and its cube root is
@@ -47,6 +48,11 @@ constexpr uint32_t kBlocks = kPrepTile / 2;  // base 2x2 blocks per tile side
 // PrepareKernel).
 constexpr int kTableCtas128 = 10;
 constexpr int kYuvCtas128 = 8;
+// The curve decode: as many warps of 64 registers as the YUV decode (a 4K
+// ST 2084 pair's prepare took 415 us so, 420 at six CTAs; a 4000x2667 16-bit
+// sRGB pair 398 us at eight, 424 at six and 451 at five).
+constexpr int kCurveCtas128 = 8;
+constexpr int kCurveCtas256 = 4;
 
 // The last prefix entry <= index (start[0] == 0 <= index < start[count]).
 __device__ __forceinline__ uint32_t FindSlot(const uint32_t* __restrict__ start, uint32_t count,
@@ -121,6 +127,11 @@ __device__ __forceinline__ float2 Cbrt2(float2 x) {
 
 __device__ __forceinline__ float2 Max0(float2 v) {
     return make_float2(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f));
+}
+
+// ss2dm::cbrt of both lanes, out of line.
+__device__ __noinline__ float2 SharedCbrt2(float2 x) {
+    return make_float2(ss2dm::cbrt(x.x), ss2dm::cbrt(x.y));
 }
 
 // prepare.comp:81-98 for two pixels. Only the channels in `mask` are
@@ -261,6 +272,81 @@ __device__ __forceinline__ void TableBlock(const DevSourceHead& s, const float* 
     }
 }
 
+// Xyb2<false> with one range check for all the mixes.
+__device__ __forceinline__ void XybCurve2(float2 r, float2 g, float2 b, uint32_t mask,
+                                          float2 out[3]) {
+    const auto mix = [&](float k0, float k1, float k2) {
+        const float2 m = __ffma2_rn(
+            Pack(k0), r, __ffma2_rn(Pack(k1), g, __ffma2_rn(Pack(k2), b, Pack(kBias))));
+        return Max0(m);
+    };
+    const float2 m0 = mix(kM00, kM01, kM02), m1 = mix(kM10, kM11, kM12);
+    const bool has_b = (mask & 4u) != 0;
+    const auto in_band = [](float2 v) {
+        return v.x >= kCbrtRouteLo && v.x < kCbrtRouteHi && v.y >= kCbrtRouteLo &&
+               v.y < kCbrtRouteHi;
+    };
+    const float2 m2 = has_b ? mix(kM20, kM21, kM22) : m1;
+    const bool direct = in_band(m0) && in_band(m1) && in_band(m2);
+    const float2 c0 = __fadd2_rn(direct ? Cbrt2<true>(m0) : SharedCbrt2(m0), Pack(-kCbrtBias));
+    const float2 c1 = __fadd2_rn(direct ? Cbrt2<true>(m1) : SharedCbrt2(m1), Pack(-kCbrtBias));
+    const float2 sum = __fadd2_rn(c0, c1);
+    out[0] = __ffma2_rn(__fmul2_rn(Pack(0.5f), __fadd2_rn(c0, Neg(c1))), Pack(14.0f), Pack(0.42f));
+    out[1] = __ffma2_rn(Pack(0.5f), sum, Pack(0.01f));
+    out[2] = Pack(0.0f);
+    if (has_b) {
+        const float2 c2 = __fadd2_rn(direct ? Cbrt2<true>(m2) : SharedCbrt2(m2), Pack(-kCbrtBias));
+        out[2] = __fadd2_rn(__ffma2_rn(Pack(-0.5f), sum, c2), Pack(0.55f));
+    }
+}
+
+// A curve image's base block (bx, by), row by row (one copy of the row's
+// code: unrolled, the transfers' bodies would not fit the instruction caches):
+// stores level 0 and leaves the block's sums, in BoxAverage's order, in sum[0].
+template <bool kHalf>
+__device__ __forceinline__ void CurveBlock(const DevSourceHead& s, const CurveWords& cw,
+                                           const float* stage, int plane, const CurveTables& tab,
+                                           uint32_t gx, uint32_t gy, uint32_t hx, uint32_t bx,
+                                           uint32_t by, const LevelInfo& lv, uint32_t mask0,
+                                           float (&sum)[4][3]) {
+    const uint32_t x0 = 2 * bx, y0 = 2 * by;
+    float e[4][3];
+    if (s.chroma_variant) {
+        ChromaFromStage(s, stage, plane, gx, gy, x0, y0, e);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) e[i][1] = e[i][2] = 0.0f;
+    }
+    float2 top[3] = {Pack(0.0f), Pack(0.0f), Pack(0.0f)};
+#pragma unroll 1
+    for (uint32_t h = 0; h < 2; ++h) {
+        float2 q[3];
+        CurveRow(s, cw, tab, hx, h, x0, y0 + h,
+                 make_float2(h ? e[2][1] : e[0][1], h ? e[3][1] : e[1][1]),
+                 make_float2(h ? e[2][2] : e[0][2], h ? e[3][2] : e[1][2]), q);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            sum[0][c] = h ? __fadd_rn(__fadd_rn(sum[0][c], q[c].x), q[c].y)
+                          : __fadd_rn(q[c].x, q[c].y);
+        if (!mask0) continue;
+        float2 row[3];
+        XybCurve2(q[0], q[1], q[2], mask0, row);
+        if (h == 0) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) top[c] = row[c];
+            continue;
+        }
+        const bool two = x0 + 1 < s.width, second_row = y0 + 1 < s.height;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (!(mask0 & (1u << c))) continue;
+            PutBlock<kHalf>(lv.plane[0][c], PlaneIndex(lv.pitch[0], x0, y0), top[c].x,
+                            second_row ? row[c].x : 0.0f, two ? top[c].y : 0.0f,
+                            two && second_row ? row[c].y : 0.0f);
+        }
+    }
+}
+
 // CTAs per SM: five of 256 threads (40 warps) for the table and YUV
 // decodes, four for the generic one; the table decode also runs as ten CTAs
 // of 128 threads (see LaunchPrepareOf). The decodes' long dependency chains
@@ -276,9 +362,12 @@ __device__ __forceinline__ void TableBlock(const DevSourceHead& s, const float* 
 #define VQM_YUV_PREPARE_CTAS 5
 #endif
 template <int kGroup, bool kHalf, int kNT>
-__global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCtas128 : kYuvCtas128)
+__global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0   ? kTableCtas128
+                                                              : kGroup == 3 ? kCurveCtas128
+                                                                            : kYuvCtas128)
                                        : kGroup == 0 ? 5
                                        : kGroup == 1 ? VQM_YUV_PREPARE_CTAS
+                                       : kGroup == 3 ? kCurveCtas256
                                                      : VQM_GENERIC_PREPARE_CTAS)
     PrepareKernel(DevBatch batch) {
     constexpr uint32_t kThreads = kNT;
@@ -286,6 +375,7 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
     constexpr uint32_t kRowPasses = kBlocks / kRows;  // 2 or 4
     constexpr bool kTable = kGroup == 0;  // 8-bit RGB/grey by table
     constexpr bool kYuv = kGroup == 1;    // yuv_fast images
+    constexpr bool kCurve = kGroup == 3;  // curve images
     // Level-1 tile (32x32) of each channel, then the levels after it in two
     // alternating buffers: odd levels in `ladder_a`, even ones in `ladder_b`.
     __shared__ __align__(16) float ladder_a[3][kBlocks * kBlocks];
@@ -298,9 +388,10 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
     // power's tables.
     // The 128-thread YUV kernel stages 4:2:0 windows only (the host sends
     // it launches whose images all have 4:2:0 chroma or none subsampled).
-    constexpr int kStagePlane = (kYuv && kNT == 128) ? kChromaStage420 : kChromaStage;
-    __shared__ float chroma_stage[kYuv ? 2 * kStagePlane : 1];
+    constexpr int kStagePlane = kNT == 128 ? kChromaStage420 : kChromaStage;
+    __shared__ float chroma_stage[kYuv || kCurve ? 2 * kStagePlane : 1];
     __shared__ float pow_table[kYuv ? PowTable::kFloats : 1];
+    __shared__ std::conditional_t<kCurve, CurveTables, char> curve_tables;
 
     const uint32_t tid = threadIdx.x;
     const uint32_t n_items = batch.prep_items[kGroup];
@@ -335,6 +426,7 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
             pow_table[PowTable::kExpHi + tid] = e.x;
             pow_table[PowTable::kExpLo + tid] = e.y;
         }
+        if constexpr (kCurve) StageCurveTables(curve_tables);
         if (tid < kMaxLevels * 3) {
             const uint32_t l = tid / 3, c = tid % 3;
             const bool kept = l < P.levels && (P.mask[l] & (1u << c));
@@ -356,6 +448,8 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
             uint32_t ok = 1;
             for (int c = 0; c < (ps.family == 0 ? 1 : 3); ++c)
                 ok &= ((reinterpret_cast<uintptr_t>(ps.plane[c]) | ps.row_bytes[c]) & 3u) == 0;
+            if (kCurve && ps.alpha)
+                ok &= ((reinterpret_cast<uintptr_t>(ps.plane[3]) | ps.row_bytes[3]) & 3u) == 0;
             aligned4 = ok;
         }
     }
@@ -365,8 +459,8 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
     const auto body = [=](auto in_range) {
     constexpr bool kInRange = decltype(in_range)::value;
     const DevSourceHead& s = src_s;
-    if constexpr (kYuv) {
-        if (s.chroma_variant) {
+    if constexpr (kYuv || kCurve) {
+        if (s.chroma_variant && s.family == 2) {
             // A window larger than the stage would overrun it: such an image
             // never reaches this kernel, and if it did its tiles are left
             // unwritten rather than read out of bounds.
@@ -410,6 +504,8 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
             }
         }
         float l1[2][3];
+        [[maybe_unused]] CurveWords cw;
+        if constexpr (kCurve) LoadCurveWords(s, aligned4 != 0, 2 * bx0, 2 * by, cw);
         // Unrolled for the table decode (the words and averages stay in
         // registers); rolled for the generic decode, whose body is large.
 #pragma unroll(kTable ? 2 : 1)
@@ -426,7 +522,10 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
                                         0.0f, 0.0f, 0.0f, 0.0f);
             }
             if (in_block) {
-                if constexpr (kTable) {
+                if constexpr (kCurve) {
+                    CurveBlock<kHalf>(s, cw, chroma_stage, kStagePlane, curve_tables, gx,
+                                                gy, hx, bx, by, lv, mask0, lin);
+                } else if constexpr (kTable) {
                     TableBlock(s, lut, fast, w4, hx, bx, by, lin);
                 } else if constexpr (kYuv) {
                     // Even width and height (PrepGroup): the block is whole.
@@ -438,7 +537,7 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
                 // Level 0: the block is one aligned float4 of the row-pair
                 // plane, (x0, y0), (x0, y0+1), (x0+1, y0), (x0+1, y0+1); a
                 // column or row past the image is the plane's zero padding.
-                if (mask0) {
+                if (!kCurve && mask0) {
                     float2 top[3], bottom[3];
                     Xyb2<kInRange>(make_float2(lin[0][0], lin[1][0]),
                                    make_float2(lin[0][1], lin[1][1]),
@@ -461,7 +560,8 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
             float avg[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                avg[c] = BoxAverage<kHalf>(lin[0][c], lin[1][c], lin[2][c], lin[3][c]);
+                avg[c] = kCurve ? PlaneRound<kHalf>(__fmul_rn(lin[0][c], 0.25f))
+                                : BoxAverage<kHalf>(lin[0][c], lin[1][c], lin[2][c], lin[3][c]);
             // Register copies, not an index, for the rolled form.
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -563,7 +663,7 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0 ? kTableCta
         }
     }
     };
-    if (src_s.in_range) body(std::true_type{});
+    if (!kCurve && src_s.in_range) body(std::true_type{});
     else body(std::false_type{});
 }
 
@@ -577,6 +677,8 @@ cudaError_t PreloadPrepareOf() {
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<1, kHalf, 256>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<1, kHalf, 128>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<2, kHalf, 256>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<3, kHalf, 256>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<3, kHalf, 128>);
     return e;
 }
 cudaError_t PreloadPrepare() {
@@ -671,12 +773,22 @@ void LaunchPrepareOf(const DevBatch& b, cudaStream_t stream) {
     // chroma: eight 128-thread CTAs per SM with the smaller window (uneven
     // prepare 5.76 -> 5.56 ms).
     if (b.prep_blocks[1]) {
-        if (b.yuv420 && b.prep_blocks[1] >= 2u * 5u * DeviceSmCount())
+        if ((b.windows420 & kWindowsYuv) && b.prep_blocks[1] >= 2u * 5u * DeviceSmCount())
             PrepareKernel<1, kHalf, 128><<<b.prep_blocks[1], 128, 0, stream>>>(b);
         else
             PrepareKernel<1, kHalf, 256><<<b.prep_blocks[1], 256, 0, stream>>>(b);
     }
     if (b.prep_blocks[2]) PrepareKernel<2, kHalf, 256><<<b.prep_blocks[2], 256, 0, stream>>>(b);
+    // The curve decode by the same rule (two waves of its 256-thread CTAs).
+    // Against the generic kernel, which these images ran before: 4K ST 2084
+    // 4:2:0 831 -> 415 us a pair, 1080p HLG 4:2:0 151 -> 70, 4000x2667 16-bit
+    // sRGB 628 -> 400, 1001x667 8-bit sRGB with alpha 47 -> 32.
+    if (b.prep_blocks[3]) {
+        if ((b.windows420 & kWindowsCurve) && b.prep_blocks[3] >= 2u * 4u * DeviceSmCount())
+            PrepareKernel<3, kHalf, 128><<<b.prep_blocks[3], 128, 0, stream>>>(b);
+        else
+            PrepareKernel<3, kHalf, 256><<<b.prep_blocks[3], 256, 0, stream>>>(b);
+    }
 }
 cudaError_t LaunchPrepare(const DevBatch& b, cudaStream_t stream) {
     if (b.half)

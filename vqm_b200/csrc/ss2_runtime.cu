@@ -994,14 +994,14 @@ private:
         const DevPair* hp = mem_.HostPair(0);
         const uint8_t g0 = static_cast<uint8_t>(PrepGroup(hp->src[0]));
         const uint8_t g1 = static_cast<uint8_t>(PrepGroup(hp->src[1]));
-        // The YUV prepare kernel (and its window) depends on the images'
-        // chroma subsampling too.
-        bool yuv420 = true;
-        for (int k = skip_original ? 1 : 0; k < 2; ++k)
-            if (PrepGroup(hp->src[k]) == 1 && !Yuv420Window(hp->src[k])) yuv420 = false;
-        mem_.dev.yuv420 = yuv420 ? 1u : 0u;
-        const int key = g0 + kPrepGroups * (g1 + kPrepGroups * ((skip_original ? 1 : 0) +
-                                                                 2 * (yuv420 ? 1 : 0)));
+        // The YUV and curve prepare kernels (and their window) depend on the
+        // images' chroma subsampling too.
+        uint32_t windows = kWindowsYuv | kWindowsCurve;
+        if (!skip_original) windows &= ~LargeWindow(hp->src[0], g0);
+        windows &= ~LargeWindow(hp->src[1], g1);
+        mem_.dev.windows420 = windows;
+        const uint32_t key =
+            g0 + kPrepGroups * (g1 + kPrepGroups * ((skip_original ? 1u : 0u) + 2u * windows));
         BuildPrepLists(tables_, {{g0, g1}}, skip_original);
         mem_.StagePrep(tables_);
         const size_t upload = mem_.head_bytes;
@@ -1042,7 +1042,7 @@ private:
     int device_ = 0;
     cudaStream_t own_stream_ = nullptr, stream_ = nullptr;
     cudaEvent_t done_ = nullptr, copied_ = nullptr;
-    cudaGraphExec_t graph_exec_[4 * kPrepGroups * kPrepGroups] = {};
+    cudaGraphExec_t graph_exec_[8 * kPrepGroups * kPrepGroups] = {};
     bool reference_valid_ = false;
     uint64_t reference_handle_ = 0;
     float reference_background_ = 0.0f;
@@ -1197,14 +1197,13 @@ public:
             }
         }
         PrepGroups group(n);
-        bool yuv420 = true;
+        uint32_t windows = kWindowsYuv | kWindowsCurve;
         for (uint32_t i = 0; i < n; ++i) {
             group[i] = {static_cast<uint8_t>(PrepGroup(t.pairs[i].src[0])),
                         static_cast<uint8_t>(PrepGroup(t.pairs[i].src[1]))};
-            for (int k = 0; k < 2; ++k)
-                if (group[i][k] == 1 && !Yuv420Window(t.pairs[i].src[k])) yuv420 = false;
+            for (int k = 0; k < 2; ++k) windows &= ~LargeWindow(t.pairs[i].src[k], group[i][k]);
         }
-        mem_.dev.yuv420 = yuv420 ? 1u : 0u;
+        mem_.dev.windows420 = windows;
         BuildPrepLists(t, group);
         mem_.Stage(t);
         if (host_bytes) VQM_CK(cudaEventRecord(copied_, stream_));
