@@ -227,6 +227,19 @@ __device__ __forceinline__ void IssueTileLoadsHalf(unsigned char* staging, const
     }
 }
 
+// Chunk q of a row pair of the binary16 window as floats of the row pair `row`.
+template <int TW, int TH, int NT>
+__device__ __forceinline__ void WidenChunk(const uint4& v, float* row, int q) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int col = 4 * q + i - 2;  // float window column (x0 - 6 based)
+        if (col < 0 || col >= Tile<TW, TH, NT>::SW) continue;
+        const __half2 h = *reinterpret_cast<const __half2*>(&w[i]);
+        *reinterpret_cast<float2*>(row + 2 * col) = __half22float2(h);
+    }
+}
+
 // The staged binary16 window to the float row-pair window of `src`.
 template <int TW, int TH, int NT>
 __device__ __forceinline__ void ConvertHalfTile(const unsigned char* staging, float* src) {
@@ -236,18 +249,65 @@ __device__ __forceinline__ void ConvertHalfTile(const unsigned char* staging, fl
         const int img = k >= H::CHUNKS ? 1 : 0;
         const int kk = k - img * H::CHUNKS;
         const int rp = kk / H::CQ, q = kk - rp * H::CQ;
-        const uint4 v = *reinterpret_cast<const uint4*>(staging + 16 * k);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        float* row = src + img * T::IMG + rp * T::SRS;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int col = 4 * q + i - 2;  // float window column (x0 - 6 based)
-            if (col < 0 || col >= T::SW) continue;
-            const __half2 h = *reinterpret_cast<const __half2*>(&w[i]);
-            *reinterpret_cast<float2*>(row + 2 * col) = __half22float2(h);
-        }
+        WidenChunk<TW, TH, NT>(*reinterpret_cast<const uint4*>(staging + 16 * k),
+                               src + img * T::IMG + rp * T::SRS, q);
     }
 }
+
+// Half planes in a strip: there is no room to stage the next tile's window
+// while the horizontal planes are live, so a thread holds its 16-byte chunks
+// (4 columns x 2 rows of an image) in registers between the load and the
+// widening store. The chunks are the window's from row pair `rp_begin` on,
+// both images'. (32 1080p pairs: blur 1.24 ms with a tile per CTA, which
+// stages the chunks in the free horizontal planes, 1.00 ms with strips; float
+// planes take 0.78.)
+template <int TW, int TH, int NT>
+struct HalfChunks {
+    using T = Tile<TW, TH, NT>;
+    using H = HalfWindow<TW, TH, NT>;
+    static constexpr int kMost = (2 * H::CHUNKS + NT - 1) / NT;
+    uint4 v[kMost];
+
+    // Chunk k of a window that starts at row pair `rp_begin`.
+    static __device__ __forceinline__ void At(int k, int rp_begin, int& img, int& rp, int& q) {
+        const int per_image = (T::RP - rp_begin) * H::CQ;
+        img = k >= per_image ? 1 : 0;
+        const int kk = k - img * per_image;
+        rp = kk / H::CQ;
+        q = kk - rp * H::CQ;
+        rp += rp_begin;
+    }
+    __device__ __forceinline__ void Load(const TileRef& t, int rp_begin) {
+        const uint32_t wq = static_cast<uint32_t>(t.w + 3) >> 2;
+        const uint32_t hp = static_cast<uint32_t>(t.h + 1) >> 1;
+        const int cq0 = (t.x0 >> 2) - 2, ry0 = (t.y0 >> 1) - kRadius / 2;
+        const int count = 2 * (T::RP - rp_begin) * H::CQ;
+#pragma unroll
+        for (int i = 0; i < kMost; ++i) {
+            const int k = static_cast<int>(threadIdx.x) + i * NT;
+            v[i] = make_uint4(0, 0, 0, 0);
+            if (k >= count) continue;
+            int img, rp, q;
+            At(k, rp_begin, img, rp, q);
+            const int gy = ry0 + rp, gq = cq0 + q;
+            if (static_cast<uint32_t>(gy) < hp && static_cast<uint32_t>(gq) < wq)
+                v[i] = __ldg(reinterpret_cast<const uint4*>(
+                    reinterpret_cast<const __half*>(img ? t.pb : t.pa) +
+                    (static_cast<uint32_t>(gy) * t.pitch + 8u * static_cast<uint32_t>(gq))));
+        }
+    }
+    __device__ __forceinline__ void Store(float* src, int rp_begin) const {
+        const int count = 2 * (T::RP - rp_begin) * H::CQ;
+#pragma unroll
+        for (int i = 0; i < kMost; ++i) {
+            const int k = static_cast<int>(threadIdx.x) + i * NT;
+            if (k >= count) continue;
+            int img, rp, q;
+            At(k, rp_begin, img, rp, q);
+            WidenChunk<TW, TH, NT>(v[i], src + img * T::IMG + rp * T::SRS, q);
+        }
+    }
+};
 
 __device__ __forceinline__ float2 Pack(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 Neg(float2 v) { return make_float2(-v.x, -v.y); }
@@ -730,7 +790,7 @@ __device__ __forceinline__ void MoveHalo(float* hq) {
 }
 
 // Strip `block` of the launch (blur_start counts strips).
-template <int TW, int TH, int NT, int S>
+template <int TW, int TH, int NT, int S, bool kHalf = false>
 __device__ __forceinline__ void RunStrip(const DevBatch& batch, uint32_t block, float* src,
                                          float* hq) {
     const uint32_t si = FindSlot(batch.blur_start, batch.segments, block);
@@ -740,14 +800,20 @@ __device__ __forceinline__ void RunStrip(const DevBatch& batch, uint32_t block, 
     const uint32_t tiles_y = seg.tiles / seg.tiles_x;
     const uint32_t ty0 = sy * S;
     const int count = static_cast<int>(min(static_cast<uint32_t>(S), tiles_y - ty0));
-    TileRef t = SegmentTile<TW, TH>(batch, seg, si, strip - sy * seg.tiles_x, ty0);
-    IssueTileLoads<TW, TH, NT>(src, t);
-    CpAsyncCommit();
+    TileRef t = SegmentTile<TW, TH, kHalf>(batch, seg, si, strip - sy * seg.tiles_x, ty0);
+    if constexpr (kHalf) {
+        HalfChunks<TW, TH, NT> chunks;
+        chunks.Load(t, 0);
+        chunks.Store(src, 0);
+    } else {
+        IssueTileLoads<TW, TH, NT>(src, t);
+        CpAsyncCommit();
+    }
     float2 sum[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) sum[i] = make_float2(0.0f, 0.0f);
     for (int k = 0; k < count; ++k) {
-        CpAsyncWait<0>();
+        if constexpr (!kHalf) CpAsyncWait<0>();
         __syncthreads();
         HorizontalPass<TW, TH, NT>(batch.taps2, src, hq, k == 0 ? 0 : kRadius);
         __syncthreads();
@@ -758,9 +824,16 @@ __device__ __forceinline__ void RunStrip(const DevBatch& batch, uint32_t block, 
         __syncthreads();  // every read of the window and of `hq` is done
         if (k + 1 < count) {
             t.y0 += TH;
-            IssueTileLoads<TW, TH, NT>(src, t, kRadius / 2);
-            CpAsyncCommit();
-            MoveHalo<TW, TH, NT>(hq);
+            if constexpr (kHalf) {
+                HalfChunks<TW, TH, NT> chunks;
+                chunks.Load(t, kRadius / 2);
+                MoveHalo<TW, TH, NT>(hq);
+                chunks.Store(src, kRadius / 2);
+            } else {
+                IssueTileLoads<TW, TH, NT>(src, t, kRadius / 2);
+                CpAsyncCommit();
+                MoveHalo<TW, TH, NT>(hq);
+            }
         }
     }
     ReducePartials<NT>(sum, HqScratch<TW, TH, NT>{hq},
@@ -768,12 +841,12 @@ __device__ __forceinline__ void RunStrip(const DevBatch& batch, uint32_t block, 
     FinishSegment<NT>(batch, si, reinterpret_cast<double*>(src));
 }
 
-template <int TW, int TH, int NT, int MB, int S>
+template <int TW, int TH, int NT, int MB, int S, bool kHalf = false>
 __global__ void __launch_bounds__(NT, MB) Ss2BlurStripKernel(DevBatch batch) {
     using T = Tile<TW, TH, NT>;
     extern __shared__ __align__(16) unsigned char smem[];
-    RunStrip<TW, TH, NT, S>(batch, blockIdx.x, reinterpret_cast<float*>(smem),
-                            reinterpret_cast<float*>(smem + T::kSrcBytes));
+    RunStrip<TW, TH, NT, S, kHalf>(batch, blockIdx.x, reinterpret_cast<float*>(smem),
+                                   reinterpret_cast<float*>(smem + T::kSrcBytes));
 }
 
 // A tile queue: as many CTAs as the device holds at once, each taking the
@@ -903,16 +976,21 @@ cudaError_t LaunchQueue(const DevBatch& b, cudaStream_t stream, bool launch) {
     return cudaGetLastError();
 }
 
-template <int TW, int TH, int NT, int MB, int S>
-cudaError_t LaunchStrips(const DevBatch& b, cudaStream_t stream, bool launch) {
+template <int TW, int TH, int NT, int MB, int S, bool kHalf>
+cudaError_t LaunchStripsAs(const DevBatch& b, cudaStream_t stream, bool launch) {
     using T = Tile<TW, TH, NT>;
     static LaunchCache cache;
     constexpr size_t smem = T::kSrcBytes + T::kHqBytes;
     const cudaError_t e =
-        Prepare(Ss2BlurStripKernel<TW, TH, NT, MB, S>, smem, cache, NT, false, nullptr);
+        Prepare(Ss2BlurStripKernel<TW, TH, NT, MB, S, kHalf>, smem, cache, NT, false, nullptr);
     if (e != cudaSuccess || !launch) return e;
-    Ss2BlurStripKernel<TW, TH, NT, MB, S><<<b.blur_blocks, NT, smem, stream>>>(b);
+    Ss2BlurStripKernel<TW, TH, NT, MB, S, kHalf><<<b.blur_blocks, NT, smem, stream>>>(b);
     return cudaGetLastError();
+}
+template <int TW, int TH, int NT, int MB, int S>
+cudaError_t LaunchStrips(const DevBatch& b, cudaStream_t stream, bool launch) {
+    return b.half ? LaunchStripsAs<TW, TH, NT, MB, S, true>(b, stream, launch)
+                  : LaunchStripsAs<TW, TH, NT, MB, S, false>(b, stream, launch);
 }
 
 cudaError_t Dispatch(const DevBatch& b, int variant, cudaStream_t stream, bool launch) {
@@ -1007,7 +1085,8 @@ cudaError_t SetConstants(const double* weights108) {
 
 cudaError_t LaunchBlur(const DevBatch& b, int variant, cudaStream_t stream) {
     if (b.blur_blocks == 0) return cudaSuccess;
-    // Half planes run the one-tile-per-CTA kernel of the same tile shape.
+    // Half planes have no persistent kernels: the one-tile-per-CTA kernel of
+    // the same tile shape runs instead.
     if (b.half) variant = HalfPlaneVariant(variant);
     if (variant < 0) return cudaErrorInvalidValue;
     return Dispatch(b, variant, stream, true);
@@ -1029,7 +1108,7 @@ cudaError_t PreloadBlur() {
 int HalfPlaneVariant(int variant) {
     if (variant < 0 || variant >= kBlurVariantCount) return -1;
     const auto one_tile = [](const BlurVariant& v) { return !v.persistent && v.strip == 1; };
-    if (one_tile(kBlurVariants[variant])) return variant;
+    if (!kBlurVariants[variant].persistent) return variant;
     for (int i = 0; i < kBlurVariantCount; ++i)
         if (one_tile(kBlurVariants[i]) && kBlurVariants[i].w == kBlurVariants[variant].w &&
             kBlurVariants[i].h == kBlurVariants[variant].h)

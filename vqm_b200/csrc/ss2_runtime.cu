@@ -616,9 +616,8 @@ public:
         stream_ = own_stream_;
         VQM_CK(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming));
         VQM_CK(cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming));
-        if (!cfg.half_planes)
-            shape_ = BlurShape::Of(
-                AutoBlurVariant(DefaultTileGrids({{cfg.width, cfg.height}}), DeviceSms(device_)));
+        shape_ = BlurShape::Of(
+            AutoBlurVariant(DefaultTileGrids({{cfg.width, cfg.height}}), DeviceSms(device_)));
         tables_ = BuildTables({{cfg.width, cfg.height}}, shape_);
         BuildPrepLists(tables_, {{0, 0}});
         mem_.Layout(tables_);
@@ -1091,15 +1090,15 @@ public:
             shape_ = BlurShape::Of(found);
         }
         if (cfg.half_planes) {
-            // Half planes run the one-tile-per-CTA blur of the same tile (the
-            // default tile when there is none), and the tables count its
-            // blocks.
+            // Half planes run the one-tile-per-CTA blur in place of a
+            // persistent one (of the default tile when there is none of its
+            // tile), and the tables count its blocks.
             mem_.elem_bytes = 2;
             const int v = HalfPlaneVariant(shape_.variant);
             shape_ = BlurShape::Of(v < 0 ? kDefaultBlurVariant : v);
         }
         // No variant chosen: each submit picks one for its tile count.
-        auto_shape_ = !cfg.variant && !cfg.tile_w && !cfg.tile_h && !cfg.half_planes;
+        auto_shape_ = !cfg.variant && !cfg.tile_w && !cfg.tile_h;
         device_ = ResolveDevice(cfg.device);
         EnsureDevice(device_);
         VQM_CK(cudaSetDevice(device_));
