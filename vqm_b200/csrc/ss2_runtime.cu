@@ -246,10 +246,11 @@ Tables BuildTables(const std::vector<std::pair<uint32_t, uint32_t>>& sizes, Blur
     t.pairs.resize(sizes.size());
     t.blur_start.push_back(0);
     uint64_t prep = 0, blur = 0;
+    ScalePlan plan;
     for (size_t i = 0; i < sizes.size(); ++i) {
         DevPair& P = t.pairs[i];
         std::memset(static_cast<void*>(&P), 0, sizeof(DevPair));
-        const ScalePlan plan = PlanScales(sizes[i].first, sizes[i].second);
+        if (i == 0 || sizes[i] != sizes[i - 1]) plan = PlanScales(sizes[i].first, sizes[i].second);
         P.levels = static_cast<uint32_t>(plan.count);
         size_t floats = 0;
         for (int l = 0; l < plan.count; ++l) {
@@ -303,8 +304,10 @@ std::vector<std::pair<uint32_t, uint32_t>> DefaultTileGrids(
     int tw = 0, th = 0;
     BlurTileShape(kDefaultBlurVariant, &tw, &th);
     std::vector<std::pair<uint32_t, uint32_t>> grids;
-    for (const auto& wh : sizes) {
-        const ScalePlan plan = PlanScales(wh.first, wh.second);
+    ScalePlan plan;
+    for (size_t i = 0; i < sizes.size(); ++i) {
+        const auto& wh = sizes[i];
+        if (i == 0 || wh != sizes[i - 1]) plan = PlanScales(wh.first, wh.second);
         for (int l = 0; l < plan.count; ++l)
             for (int c = 0; c < 3; ++c)
                 if (plan.mask[l] & (1u << c))
@@ -1172,12 +1175,20 @@ public:
         mem_.Layout(t);
         inputs_.ensure(std::max<size_t>(host_bytes, 256));
         size_t cursor = 0;
+        const DevSource* last = nullptr;  // the previous image's, and its format
+        vqm_cu_format last_format{};
         for (uint32_t i = 0; i < n; ++i) {
             const vqm_cu_image* imgs[2] = {&o[i], &d[i]};
             for (int k = 0; k < 2; ++k) {
                 DevSource& src = t.pairs[i].src[k];
                 const vqm_cu_image& img = *imgs[k];
-                BuildSourceConstants(img.format, cfg_.chroma_filter, bg, src);
+                // A list of one format has one set of constants.
+                if (last && std::memcmp(&last_format, &img.format, sizeof(last_format)) == 0)
+                    src = *last;
+                else
+                    BuildSourceConstants(img.format, cfg_.chroma_filter, bg, src);
+                last = &src;
+                last_format = img.format;
                 const char* name = k == 0 ? "original" : "distorted";
                 if (img.memory == VQM_CU_MEMORY_HOST) {
                     uint8_t* dst = inputs_.as<uint8_t>() + cursor;
