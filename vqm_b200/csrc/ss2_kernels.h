@@ -16,6 +16,11 @@ namespace vqm_b200 {
 cudaError_t SetConstants(const double* weights108);
 
 cudaError_t LaunchPrepare(const DevBatch& batch, cudaStream_t stream);
+// The prepare of one pair whose record travels in the launch: `images` has,
+// per prepare group, a bit for each image of the pair to prepare with it. Of
+// `batch` only half and windows420 are read.
+cudaError_t LaunchPrepareOne(const DevBatch& batch, const DevPair& pair,
+                             const uint32_t (&images)[kPrepGroups], cudaStream_t stream);
 // `variant` indexes the blur kernels compiled in (BlurTileShape gives each
 // one's output tile); the batch's segments must have been tiled with it.
 // The blur also finishes every pair: its last CTA per segment sums the
@@ -53,8 +58,8 @@ uint32_t BlurBlocks(int index, uint32_t tiles_x, uint32_t tiles_y);
 // estimated time (ss2_blur.cu). A strip regroups the compensated partial
 // sums, so the choice moves a result by rounding only (~1e-7 relative).
 int AutoBlurVariant(const std::vector<std::pair<uint32_t, uint32_t>>& grids, int sms);
-// The one-tile-per-CTA variant with variant's tile shape (the variant
-// itself when it is one), which half planes run; -1 when there is none.
+// The variant half planes run for `variant`: itself, or for a persistent one
+// the one-tile-per-CTA variant of its tile shape; -1 when there is none.
 int HalfPlaneVariant(int variant);
 // The variant used when a caller does not choose one.
 constexpr int kDefaultBlurVariant = 0;

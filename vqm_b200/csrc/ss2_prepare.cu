@@ -361,15 +361,12 @@ __device__ __forceinline__ void CurveBlock(const DevSourceHead& s, const CurveWo
 #ifndef VQM_YUV_PREPARE_CTAS
 #define VQM_YUV_PREPARE_CTAS 5
 #endif
+template <int kGroup, int kNT>
+constexpr int kPrepareCtas = kNT == 128 ? (kGroup == 0 ? kTableCtas128 : kGroup == 3 ? kCurveCtas128 : kYuvCtas128) : kGroup == 0 ? 5 : kGroup == 1 ? VQM_YUV_PREPARE_CTAS : kGroup == 3 ? kCurveCtas256 : VQM_GENERIC_PREPARE_CTAS;
+
+// Tile t of one image of pair P.
 template <int kGroup, bool kHalf, int kNT>
-__global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0   ? kTableCtas128
-                                                              : kGroup == 3 ? kCurveCtas128
-                                                                            : kYuvCtas128)
-                                       : kGroup == 0 ? 5
-                                       : kGroup == 1 ? VQM_YUV_PREPARE_CTAS
-                                       : kGroup == 3 ? kCurveCtas256
-                                                     : VQM_GENERIC_PREPARE_CTAS)
-    PrepareKernel(DevBatch batch) {
+__device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_t t) {
     constexpr uint32_t kThreads = kNT;
     constexpr uint32_t kRows = kThreads / 16;         // block rows per pass
     constexpr uint32_t kRowPasses = kBlocks / kRows;  // 2 or 4
@@ -394,19 +391,8 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0   ? kTableC
     __shared__ std::conditional_t<kCurve, CurveTables, char> curve_tables;
 
     const uint32_t tid = threadIdx.x;
-    const uint32_t n_items = batch.prep_items[kGroup];
-    uint32_t before = 0;  // images in the groups ahead of this one
-#pragma unroll
-    for (int g = 0; g < kGroup; ++g) before += batch.prep_items[g];
-    const DevPrepItem* items = batch.prep_item + before;
-    const uint32_t* start = batch.prep_start + before + kGroup;
-    const uint32_t it = FindSlot(start, n_items, blockIdx.x);
-    const DevPrepItem item = items[it];
-    const DevPair& P = batch.pair[item.pair];
-    const uint32_t t = blockIdx.x - __ldg(&start[it]);
     const uint32_t gy = t / P.prep_tiles_x;
     const uint32_t gx = t - gy * P.prep_tiles_x;
-    const int image = static_cast<int>(item.image);
 
     {
         const uint32_t* from = reinterpret_cast<const uint32_t*>(&P.src[image]);
@@ -667,18 +653,50 @@ __global__ void __launch_bounds__(kNT, kNT == 128     ? (kGroup == 0   ? kTableC
     else body(std::false_type{});
 }
 
+// A batch's images: each CTA finds its tile in the group's prefix offsets.
+template <int kGroup, bool kHalf, int kNT>
+__global__ void __launch_bounds__(kNT, kPrepareCtas<kGroup, kNT>) PrepareKernel(DevBatch batch) {
+    const uint32_t n_items = batch.prep_items[kGroup];
+    uint32_t before = 0;  // images in the groups ahead of this one
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g) before += batch.prep_items[g];
+    const DevPrepItem* items = batch.prep_item + before;
+    const uint32_t* start = batch.prep_start + before + kGroup;
+    const uint32_t it = FindSlot(start, n_items, blockIdx.x);
+    const DevPrepItem item = items[it];
+    PrepareTile<kGroup, kHalf, kNT>(batch.pair[item.pair], static_cast<int>(item.image),
+                                    blockIdx.x - __ldg(&start[it]));
+}
+
+// One pair, its record in the launch's parameters: nothing has to be uploaded
+// ahead of the kernel, and a CTA's first reads come from the constant bank
+// instead of a chain of dependent global loads. `images`: bit k, image k.
+template <int kGroup, bool kHalf, int kNT>
+__global__ void __launch_bounds__(kNT, kPrepareCtas<kGroup, kNT>)
+    PrepareOneKernel(const __grid_constant__ DevPair pair, uint32_t images) {
+    const uint32_t tiles = pair.prep_tiles_x * pair.prep_tiles_y;
+    const bool second = blockIdx.x >= tiles;
+    PrepareTile<kGroup, kHalf, kNT>(pair, second || images == 2u ? 1 : 0,
+                                    second ? blockIdx.x - tiles : blockIdx.x);
+}
+
 }  // namespace
 
+template <int kGroup, bool kHalf, int kNT>
+cudaError_t PreloadPrepareKernels() {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, PrepareKernel<kGroup, kHalf, kNT>);
+    return e == cudaSuccess ? cudaFuncGetAttributes(&a, PrepareOneKernel<kGroup, kHalf, kNT>) : e;
+}
 template <bool kHalf>
 cudaError_t PreloadPrepareOf() {
-    cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, PrepareKernel<0, kHalf, 256>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<0, kHalf, 128>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<1, kHalf, 256>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<1, kHalf, 128>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<2, kHalf, 256>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<3, kHalf, 256>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, PrepareKernel<3, kHalf, 128>);
+    cudaError_t e = PreloadPrepareKernels<0, kHalf, 256>();
+    if (e == cudaSuccess) e = PreloadPrepareKernels<0, kHalf, 128>();
+    if (e == cudaSuccess) e = PreloadPrepareKernels<1, kHalf, 256>();
+    if (e == cudaSuccess) e = PreloadPrepareKernels<1, kHalf, 128>();
+    if (e == cudaSuccess) e = PreloadPrepareKernels<2, kHalf, 256>();
+    if (e == cudaSuccess) e = PreloadPrepareKernels<3, kHalf, 256>();
+    if (e == cudaSuccess) e = PreloadPrepareKernels<3, kHalf, 128>();
     return e;
 }
 cudaError_t PreloadPrepare() {
@@ -756,45 +774,72 @@ static uint32_t DeviceSmCount() {
     return static_cast<uint32_t>(cached[device]);
 }
 
-template <bool kHalf>
-void LaunchPrepareOf(const DevBatch& b, cudaStream_t stream) {
+// Where a group's images are: a batch's tables, or one pair's record.
+struct PrepareBatch {
+    const DevBatch& b;
+    uint32_t Blocks(int g) const { return b.prep_blocks[g]; }
+    template <int kGroup, bool kHalf, int kNT>
+    void Launch(cudaStream_t stream) const {
+        PrepareKernel<kGroup, kHalf, kNT><<<b.prep_blocks[kGroup], kNT, 0, stream>>>(b);
+    }
+};
+struct PrepareOne {
+    const DevPair& pair;
+    const uint32_t* images;
+    uint32_t Blocks(int g) const {
+        const uint32_t n = (images[g] & 1u) + (images[g] >> 1);
+        return n * pair.prep_tiles_x * pair.prep_tiles_y;
+    }
+    template <int kGroup, bool kHalf, int kNT>
+    void Launch(cudaStream_t stream) const {
+        PrepareOneKernel<kGroup, kHalf, kNT>
+            <<<Blocks(kGroup), kNT, 0, stream>>>(pair, images[kGroup]);
+    }
+};
+
+template <bool kHalf, class Images>
+void LaunchPrepareOf(const Images& images, uint32_t windows420, cudaStream_t stream) {
     // The table decode of a launch of at least two waves of 256-thread CTAs
     // runs as ten CTAs of 128 threads per SM: 64 1080p pairs 1.149 -> 1.075
     // ms. Smaller launches keep 256 threads, which finish a CTA's tile
     // sooner (one 1080p pair 27.0 against 28.7 us, one 256x256 pair 12.3
     // against 17.0 us).
-    if (b.prep_blocks[0]) {
-        if (b.prep_blocks[0] >= 2u * 5u * DeviceSmCount())
-            PrepareKernel<0, kHalf, 128><<<b.prep_blocks[0], 128, 0, stream>>>(b);
-        else
-            PrepareKernel<0, kHalf, 256><<<b.prep_blocks[0], 256, 0, stream>>>(b);
+    if (const uint32_t n = images.Blocks(0)) {
+        if (n >= 2u * 5u * DeviceSmCount()) images.template Launch<0, kHalf, 128>(stream);
+        else images.template Launch<0, kHalf, 256>(stream);
     }
     // The YUV decode likewise, when every image of the launch has 4:2:0
     // chroma: eight 128-thread CTAs per SM with the smaller window (uneven
     // prepare 5.76 -> 5.56 ms).
-    if (b.prep_blocks[1]) {
-        if ((b.windows420 & kWindowsYuv) && b.prep_blocks[1] >= 2u * 5u * DeviceSmCount())
-            PrepareKernel<1, kHalf, 128><<<b.prep_blocks[1], 128, 0, stream>>>(b);
+    if (const uint32_t n = images.Blocks(1)) {
+        if ((windows420 & kWindowsYuv) && n >= 2u * 5u * DeviceSmCount())
+            images.template Launch<1, kHalf, 128>(stream);
         else
-            PrepareKernel<1, kHalf, 256><<<b.prep_blocks[1], 256, 0, stream>>>(b);
+            images.template Launch<1, kHalf, 256>(stream);
     }
-    if (b.prep_blocks[2]) PrepareKernel<2, kHalf, 256><<<b.prep_blocks[2], 256, 0, stream>>>(b);
+    if (images.Blocks(2)) images.template Launch<2, kHalf, 256>(stream);
     // The curve decode by the same rule (two waves of its 256-thread CTAs).
     // Against the generic kernel, which these images ran before: 4K ST 2084
     // 4:2:0 831 -> 415 us a pair, 1080p HLG 4:2:0 151 -> 70, 4000x2667 16-bit
     // sRGB 628 -> 400, 1001x667 8-bit sRGB with alpha 47 -> 32.
-    if (b.prep_blocks[3]) {
-        if ((b.windows420 & kWindowsCurve) && b.prep_blocks[3] >= 2u * 4u * DeviceSmCount())
-            PrepareKernel<3, kHalf, 128><<<b.prep_blocks[3], 128, 0, stream>>>(b);
+    if (const uint32_t n = images.Blocks(3)) {
+        if ((windows420 & kWindowsCurve) && n >= 2u * 4u * DeviceSmCount())
+            images.template Launch<3, kHalf, 128>(stream);
         else
-            PrepareKernel<3, kHalf, 256><<<b.prep_blocks[3], 256, 0, stream>>>(b);
+            images.template Launch<3, kHalf, 256>(stream);
     }
 }
 cudaError_t LaunchPrepare(const DevBatch& b, cudaStream_t stream) {
-    if (b.half)
-        LaunchPrepareOf<true>(b, stream);
-    else
-        LaunchPrepareOf<false>(b, stream);
+    const PrepareBatch images{b};
+    if (b.half) LaunchPrepareOf<true>(images, b.windows420, stream);
+    else LaunchPrepareOf<false>(images, b.windows420, stream);
+    return cudaGetLastError();
+}
+cudaError_t LaunchPrepareOne(const DevBatch& b, const DevPair& pair,
+                             const uint32_t (&images)[kPrepGroups], cudaStream_t stream) {
+    const PrepareOne one{pair, images};
+    if (b.half) LaunchPrepareOf<true>(one, b.windows420, stream);
+    else LaunchPrepareOf<false>(one, b.windows420, stream);
     return cudaGetLastError();
 }
 

@@ -4,8 +4,8 @@
 //   Pipeline  one geometry, one pair in flight: VQM's Ssimulacra2Pipeline
 //             (include/ssimulacra2.h:83-215) with CUDA in place of Vulkan.
 //             Its device tables never change after construction, so each
-//             pair is one CUDA-graph replay of [descriptor upload, prepare,
-//             blur, finalize, result read-back].
+//             pair is one CUDA-graph replay of [prepare, blur], with the
+//             pair's record in the prepare nodes' parameters.
 //   Batch     any number of pairs of any sizes and formats, scored by one
 //             launch per stage over all of them (the batched path).
 //
@@ -324,13 +324,12 @@ int DeviceSms(int device) {
 
 // Splits the images into the prepare groups (group[i][k]: PrepGroup of
 // image k of pair i) and lays out each group's prefix tile offsets. The list
-// sizes do not depend on the split. `skip_original`, when set, leaves every
-// pair's image 0 out (its pyramid is already in place).
+// sizes do not depend on the split.
 using PrepGroups = std::vector<std::array<uint8_t, 2>>;
-void BuildPrepLists(Tables& t, const PrepGroups& group, bool skip_original = false) {
+void BuildPrepLists(Tables& t, const PrepGroups& group) {
     uint32_t n[kPrepGroups] = {};
     for (size_t i = 0; i < t.pairs.size(); ++i)
-        for (int k = skip_original ? 1 : 0; k < 2; ++k) ++n[group[i][k]];
+        for (int k = 0; k < 2; ++k) ++n[group[i][k]];
     uint32_t first[kPrepGroups];   // the group's first item
     uint32_t* start[kPrepGroups];  // the group's prefix offsets
     uint32_t blocks[kPrepGroups] = {};
@@ -341,7 +340,7 @@ void BuildPrepLists(Tables& t, const PrepGroups& group, bool skip_original = fal
     }
     uint32_t at[kPrepGroups] = {};
     for (size_t i = 0; i < t.pairs.size(); ++i)
-        for (uint32_t k = skip_original ? 1 : 0; k < 2; ++k) {
+        for (uint32_t k = 0; k < 2; ++k) {
             const int g = group[i][k];
             const uint32_t pos = at[g]++;
             t.prep_items[first[g] + pos] = DevPrepItem{static_cast<uint32_t>(i), k};
@@ -634,8 +633,6 @@ public:
     ~Pipeline() {
         cudaSetDevice(device_);
         if (stream_) cudaStreamSynchronize(stream_);
-        for (auto& g : graph_exec_)
-            if (g) cudaGraphExecDestroy(g);
         if (done_) cudaEventDestroy(done_);
         if (copied_) cudaEventDestroy(copied_);
         if (own_stream_) cudaStreamDestroy(own_stream_);
@@ -985,58 +982,113 @@ private:
         return token;
     }
 
-    // [upload the pair record, prepare, blur, finalize, read back], as one
-    // graph replay when graphs are on. `skip_original` leaves the original's
-    // prepare out (its pyramid is cached).
+    // [prepare, blur with its finalize], as one graph replay when graphs are
+    // on. The pair's record goes with the prepare launches as a parameter (set
+    // anew in the graph's nodes for each submission); the blur reads only what
+    // the construction uploaded. `skip_original` leaves the original's prepare
+    // out (its pyramid is cached).
     uint64_t Launch(bool skip_original = false) {
         TraceRange trace("ss2 pipeline launch");
         if (!skip_original) reference_valid_ = false;
         // Each image's prepare group, and whether the original is prepared,
         // decide the prepare launches; one graph per combination.
         const DevPair* hp = mem_.HostPair(0);
-        const uint8_t g0 = static_cast<uint8_t>(PrepGroup(hp->src[0]));
-        const uint8_t g1 = static_cast<uint8_t>(PrepGroup(hp->src[1]));
+        const int g0 = PrepGroup(hp->src[0]), g1 = PrepGroup(hp->src[1]);
         // The YUV and curve prepare kernels (and their window) depend on the
         // images' chroma subsampling too.
         uint32_t windows = kWindowsYuv | kWindowsCurve;
-        if (!skip_original) windows &= ~LargeWindow(hp->src[0], g0);
+        uint32_t images[kPrepGroups] = {};
+        if (!skip_original) {
+            windows &= ~LargeWindow(hp->src[0], g0);
+            images[g0] |= 1u;
+        }
         windows &= ~LargeWindow(hp->src[1], g1);
+        images[g1] |= 2u;
         mem_.dev.windows420 = windows;
         const uint32_t key =
             g0 + kPrepGroups * (g1 + kPrepGroups * ((skip_original ? 1u : 0u) + 2u * windows));
-        BuildPrepLists(tables_, {{g0, g1}}, skip_original);
-        mem_.StagePrep(tables_);
-        const size_t upload = mem_.head_bytes;
         // Stream capture needs a real stream; the legacy default stream runs
         // the same work launch by launch.
         if (graphs_ && stream_ != nullptr) {
-            cudaGraphExec_t& exec = graph_exec_[key];
-            if (!exec) {
-                cudaGraph_t graph = nullptr;
-                VQM_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-                try {
-                    mem_.EnqueueUpload(upload, stream_);
-                    mem_.EnqueueKernels(shape_, stream_);
-                } catch (...) {
-                    cudaStreamEndCapture(stream_, &graph);
-                    if (graph) cudaGraphDestroy(graph);
-                    throw;
-                }
-                VQM_CK(cudaStreamEndCapture(stream_, &graph));
-                const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-                cudaGraphDestroy(graph);
-                Check(e, "cudaGraphInstantiate");
-            }
-            VQM_CK(cudaGraphLaunch(exec, stream_));
+            PairGraph& g = graphs_by_key_[key];
+            if (!g.exec) g.Capture(stream_, [&] { EnqueuePair(*hp, images); });
+            else g.SetPair(hp);
+            VQM_CK(cudaGraphLaunch(g.exec, stream_));
         } else {
-            mem_.EnqueueUpload(upload, stream_);
-            mem_.EnqueueKernels(shape_, stream_);
+            EnqueuePair(*hp, images);
         }
         VQM_CK(cudaEventRecord(done_, stream_));
         token_ = NextIncarnation();
         in_flight_ = true;
         return token_;
     }
+    void EnqueuePair(const DevPair& pair, const uint32_t (&images)[kPrepGroups]) {
+        VQM_CK(LaunchPrepareOne(mem_.dev, pair, images, stream_));
+        VQM_CK(LaunchBlur(mem_.dev, shape_.variant, stream_));
+    }
+
+    // A captured submission and its prepare nodes (the kernels that take the
+    // pair's record: one, or two where the images' groups differ).
+    struct PairGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        cudaGraphNode_t node[2] = {};
+        cudaKernelNodeParams params[2] = {};
+        uint32_t images[2] = {};
+        int nodes = 0;
+
+        PairGraph() = default;
+        PairGraph(const PairGraph&) = delete;
+        PairGraph& operator=(const PairGraph&) = delete;
+        ~PairGraph() {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+        }
+        template <class Enqueue>
+        void Capture(cudaStream_t stream, Enqueue enqueue) {
+            VQM_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+            cudaGraph_t captured = nullptr;
+            try {
+                enqueue();
+            } catch (...) {
+                cudaStreamEndCapture(stream, &captured);
+                if (captured) cudaGraphDestroy(captured);
+                throw;
+            }
+            VQM_CK(cudaStreamEndCapture(stream, &captured));
+            if (graph) cudaGraphDestroy(graph);
+            graph = captured;
+            nodes = 0;
+            // The chain in order: the prepare launches, then the blur.
+            cudaGraphNode_t at[3] = {};
+            size_t count = 0;
+            VQM_CK(cudaGraphGetNodes(graph, nullptr, &count));
+            if (count < 2 || count > 3) throw CudaFailure("cuda: unexpected graph of a pair");
+            cudaGraphNode_t root = nullptr;
+            size_t roots = 1;
+            VQM_CK(cudaGraphGetRootNodes(graph, &root, &roots));
+            at[0] = root;
+            for (size_t i = 1; i < count; ++i) {
+                size_t next = 1;
+                VQM_CK(cudaGraphNodeGetDependentNodes(at[i - 1], &at[i], &next));
+            }
+            for (size_t i = 0; i + 1 < count; ++i, ++nodes) {
+                node[i] = at[i];
+                VQM_CK(cudaGraphKernelNodeGetParams(at[i], &params[i]));
+                images[i] = *static_cast<const uint32_t*>(params[i].kernelParams[1]);
+            }
+            VQM_CK(cudaGraphInstantiate(&exec, graph, 0));
+        }
+        // The next replay's pair record.
+        void SetPair(const DevPair* pair) {
+            for (int i = 0; i < nodes; ++i) {
+                void* args[2] = {const_cast<DevPair*>(pair), &images[i]};
+                cudaKernelNodeParams p = params[i];
+                p.kernelParams = args;
+                VQM_CK(cudaGraphExecKernelNodeSetParams(exec, node[i], &p));
+            }
+        }
+    };
 
     vqm_cu_ss2_config cfg_;
     ScalePlan plan_;
@@ -1044,7 +1096,7 @@ private:
     int device_ = 0;
     cudaStream_t own_stream_ = nullptr, stream_ = nullptr;
     cudaEvent_t done_ = nullptr, copied_ = nullptr;
-    cudaGraphExec_t graph_exec_[8 * kPrepGroups * kPrepGroups] = {};
+    PairGraph graphs_by_key_[8 * kPrepGroups * kPrepGroups];
     bool reference_valid_ = false;
     uint64_t reference_handle_ = 0;
     float reference_background_ = 0.0f;
