@@ -160,16 +160,6 @@ __device__ __forceinline__ void Xyb2(float2 r, float2 g, float2 b, uint32_t mask
     }
 }
 
-// One pixel: the pair form with a duplicated lane.
-template <bool kInRange = false>
-__device__ __forceinline__ void Xyb(float r, float g, float b, uint32_t mask, float out[3]) {
-    float2 o[3];
-    Xyb2<kInRange>(Pack(r), Pack(g), Pack(b), mask, o);
-    out[0] = o[0].x;
-    out[1] = o[1].x;
-    out[2] = o[2].x;
-}
-
 // The half-plane build's rounding of a plane value (ssimu2_common.glsl:86-91).
 template <bool kHalf>
 __device__ __forceinline__ float PlaneRound(float v) {
@@ -376,7 +366,7 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
     // Level-1 tile (32x32) of each channel, then the levels after it in two
     // alternating buffers: odd levels in `ladder_a`, even ones in `ladder_b`.
     __shared__ __align__(16) float ladder_a[3][kBlocks * kBlocks];
-    __shared__ float ladder_b[3][kBlocks * kBlocks / 4];
+    __shared__ __align__(16) float ladder_b[3][kBlocks * kBlocks / 4];
     __shared__ float lut[kTable ? 256 : 1];
     __shared__ DevSourceHead src_s;  // (the byte table goes to `lut`)
     __shared__ LevelInfo lv;
@@ -592,59 +582,54 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
     if (last < 2) return;
     __syncthreads();
 
-    // Levels 2..last: the first min(side^2, NT) threads average the
-    // previous level's 2x2 blocks from the ladder (side^2 = 256, 64, 16, 4
-    // pixels; prepare.comp:149-168, clamped to the previous level's last
-    // column and row); threads that no longer take part leave, and the rest
-    // meet at a barrier of their own.
+    // Levels 2..last: the first side^2 / 2 threads average the previous
+    // level's 2x2 blocks from the ladder, two pixels of a row each (side^2 =
+    // 256, 64, 16, 4 pixels; prepare.comp:149-168): a row's four samples are
+    // one 16-byte load, and the XYB transform has a pixel in each lane. Where
+    // the previous level ends on the block's first column or row the second
+    // repeats it (the clamp to its last column and row); a pixel past the
+    // level is averaged from zeros and not stored. Threads that no longer
+    // take part leave, and the rest meet at a barrier of their own. (One
+    // pixel a thread: table prepare of 64 1080p pairs 1.149 ms, now 1.042.)
 #pragma unroll 1
     for (uint32_t level = 2; level <= last; ++level) {
-        const uint32_t shift = 6 - level;             // side = 64 >> level
-        const uint32_t side = 1u << shift;
-        const uint32_t active = side * side;
-        const uint32_t workers = active < kThreads ? active : kThreads;
+        const uint32_t shift = 5 - level;             // side / 2 = 32 >> level
+        const uint32_t side = 2u << shift;
+        const uint32_t workers = side << shift;       // side^2 / 2, at most 128
         if (tid >= workers) return;
         const uint32_t prev_side = side * 2;
-        const uint32_t pw = lv.w[level - 1], ph = lv.h[level - 1];
-        const uint32_t ox = min(gx * prev_side, pw - 1);
-        const uint32_t oy = min(gy * prev_side, ph - 1);
-        const uint32_t lx = pw - 1 - ox, ly = ph - 1 - oy;
         const float* prev0 = (level & 1u) ? &ladder_b[0][0] : &ladder_a[0][0];
         const uint32_t prev_stride = (level & 1u) ? kBlocks * kBlocks / 4 : kBlocks * kBlocks;
         float* next0 = (level & 1u) ? &ladder_a[0][0] : &ladder_b[0][0];
         const uint32_t next_stride = (level & 1u) ? kBlocks * kBlocks : kBlocks * kBlocks / 4;
-        const auto pixel = [&](uint32_t px) {
-            const uint32_t jx = px & (side - 1);
-            const uint32_t jy = px >> shift;
-            const uint32_t cx0 = min(2 * jx, lx), cx1 = min(2 * jx + 1, lx);
-            const uint32_t cy0 = min(2 * jy, ly), cy1 = min(2 * jy + 1, ly);
-            float v[3];
+        const uint32_t jx = 2 * (tid & ((1u << shift) - 1u)), jy = tid >> shift;
+        // Columns 2jx + 1 and 2jx + 3 and row 2jy + 1 of the previous level.
+        const uint32_t px = gx * prev_side + 2 * jx + 1, py = gy * prev_side + 2 * jy + 1;
+        const bool in0 = px < lv.w[level - 1], in1 = px + 2 < lv.w[level - 1];
+        const bool below = py < lv.h[level - 1];
+        const float* p = prev0 + 2 * (jy * prev_side + jx);
+        float2 v[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float* p = prev0 + c * prev_stride;
-                v[c] = BoxAverage<kHalf>(p[cy0 * prev_side + cx0], p[cy0 * prev_side + cx1],
-                                         p[cy1 * prev_side + cx0], p[cy1 * prev_side + cx1]);
-            }
-            float xyb[3];
-            Xyb<kInRange>(v[0], v[1], v[2], lv.mask[level], xyb);
-            StorePixel<kHalf>(lv, level, gx * side + jx, gy * side + jy, xyb[0], xyb[1],
-                              xyb[2]);
-            if (level < last) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) next0[c * next_stride + px] = v[c];
-            }
-        };
-        if constexpr (kThreads >= 256) {
-            pixel(tid);  // at most 256 pixels a level: one each
-        } else {
-            for (uint32_t px = tid; px < active; px += kThreads) pixel(px);
+        for (int c = 0; c < 3; ++c, p += prev_stride) {
+            const float4 t = *reinterpret_cast<const float4*>(p);
+            const float4 u = *reinterpret_cast<const float4*>(below ? p + prev_side : p);
+            v[c] = make_float2(BoxAverage<kHalf>(t.x, in0 ? t.y : t.x, u.x, in0 ? u.y : u.x),
+                               BoxAverage<kHalf>(t.z, in1 ? t.w : t.z, u.z, in1 ? u.w : u.z));
         }
+        float2 xyb[3];
+        Xyb2<kInRange>(v[0], v[1], v[2], lv.mask[level], xyb);
+        const uint32_t x = gx * side + jx, y = gy * side + jy;
+        StorePixel<kHalf>(lv, level, x, y, xyb[0].x, xyb[1].x, xyb[2].x);
+        StorePixel<kHalf>(lv, level, x + 1, y, xyb[0].y, xyb[1].y, xyb[2].y);
         if (level < last) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                *reinterpret_cast<float2*>(next0 + c * next_stride + jy * side + jx) = v[c];
             if (workers > 32) {
-                // 256, 128 or 64 threads: whole warps from warp 0.
+                // 128 threads: whole warps from warp 0.
                 asm volatile("bar.sync 1, %0;" ::"r"(workers) : "memory");
             } else {
-                __syncwarp((1u << workers) - 1u);
+                __syncwarp(workers == 32 ? 0xffffffffu : (1u << workers) - 1u);
             }
         }
     }
