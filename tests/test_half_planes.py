@@ -63,3 +63,30 @@ def test_half_plane_batch_matches_pipeline_for_every_variant():
         for g, r, (o, d) in zip(got, ref, pairs):
             bad = helpers.feature_mismatch(g.norms, r)
             assert not bad, (v, bad[:4])
+
+
+def test_half_plane_results_do_not_depend_on_the_strip_or_the_list():
+    """A half-plane blur writes one partial per tile however many tiles a CTA
+    walks down, so a pair's norms are the same bits from every strip kernel of
+    its tile shape, alone (a pipeline), and in a list long enough for the
+    longest strips."""
+    pairs = [synthetic.rgb_pair(97, 1300, 67)[:2], synthetic.rgb_pair(1280, 720, 68)[:2],
+             synthetic.yuv_pair(130, 98, 69)[:2]]
+    variants = ss2.blur_variants()
+    one_tile = {}
+    for v, (w, h, _, strip, persistent) in enumerate(variants):
+        if persistent:
+            continue
+        with ss2.Ssimulacra2Batch(variant=v, half_planes=True) as b:
+            got = [r.norms for r in b.compute_many(pairs)]
+        want = one_tile.setdefault((w, h), got)  # the one-tile kernels come first
+        assert strip > 1 or got is want
+        for g, r in zip(got, want):
+            assert np.array_equal(g, r), (v, np.max(np.abs(g - r)))
+    want = one_tile[variants[0][:2]]
+    for (o, d), r in zip(pairs, want):
+        with ss2.Ssimulacra2Pipeline(o.width, o.height, half_planes=True) as p:
+            assert np.array_equal(p.compute(o, d).norms, r)
+    with ss2.Ssimulacra2Batch(half_planes=True) as b:
+        for g, r in zip(b.compute_many([pairs[1]] * 24 + pairs), [want[1]] * 24 + want):
+            assert np.array_equal(g.norms, r)

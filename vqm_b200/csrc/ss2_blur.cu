@@ -258,8 +258,8 @@ __device__ __forceinline__ void ConvertHalfTile(const unsigned char* staging, fl
 // while the horizontal planes are live, so a thread holds its 16-byte chunks
 // (4 columns x 2 rows of an image) in registers between the load and the
 // widening store. The chunks are the window's from row pair `rp_begin` on,
-// both images'. (32 1080p pairs: blur 1.24 ms with a tile per CTA, which
-// stages the chunks in the free horizontal planes, 1.00 ms with strips; float
+// both images'. (32 1080p pairs: blur 1.22 ms with a tile per CTA, which
+// stages the chunks in the free horizontal planes, 1.03 ms with strips; float
 // planes take 0.78.)
 template <int TW, int TH, int NT>
 struct HalfChunks {
@@ -508,11 +508,11 @@ struct LinearScratch {
 
 // The CTA's six sums as one compensated partial each (scale.comp:395-436,
 // with two-sum compensation in place of the plain ladder): every thread
-// folds its two lanes, 16 lanes per sum add the block's values, and a
-// 16-lane butterfly finishes. `red(a)` is scratch array a (a < 12) of NT
-// floats. Ends with a barrier.
+// folds its two lanes (StoreSums), 16 lanes per sum add the block's values,
+// and a 16-lane butterfly finishes (FoldSums, after a barrier). `red(a)` is
+// scratch array a (a < 12) of NT floats.
 template <int NT, class Scratch>
-__device__ __forceinline__ void ReducePartials(const float2 (&sum)[6], Scratch red, double* out) {
+__device__ __forceinline__ void StoreSums(const float2 (&sum)[6], Scratch red) {
     const int tid = threadIdx.x;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -521,7 +521,10 @@ __device__ __forceinline__ void ReducePartials(const float2 (&sum)[6], Scratch r
         red(2 * k)[tid] = s;
         red(2 * k + 1)[tid] = c;
     }
-    __syncthreads();
+}
+template <int NT, class Scratch>
+__device__ __forceinline__ void FoldSums(Scratch red, double* out) {
+    const int tid = threadIdx.x;
     if (tid < 96) {  // warps 0-2, whole
         const int k = tid >> 4, i = tid & 15;
         const float* rs = red(2 * k);
@@ -537,6 +540,13 @@ __device__ __forceinline__ void ReducePartials(const float2 (&sum)[6], Scratch r
         }
         if (i == 0) out[k] = static_cast<double>(s) + static_cast<double>(c);
     }
+}
+// Both steps; ends with a barrier.
+template <int NT, class Scratch>
+__device__ __forceinline__ void ReducePartials(const float2 (&sum)[6], Scratch red, double* out) {
+    StoreSums<NT>(sum, red);
+    __syncthreads();
+    FoldSums<NT>(red, out);
     __syncthreads();
 }
 
@@ -608,8 +618,8 @@ __device__ __noinline__ void WritePairResult(const DevBatch& batch, const DevPai
     }
 }
 
-// Called by every thread of a blur CTA once its partial of segment `si` is
-// written (after a barrier). The CTA whose partial completes the segment
+// Called by every thread of a blur CTA once its `written` partials of segment
+// `si` are written (after a barrier). The CTA whose partial completes the segment
 // adds the segment's partials in FP64 in a fixed order (thread t takes
 // partials t, t + NT, ..., then a butterfly and the warps in turn), so a
 // result repeats bit for bit; the CTA whose segment completes the pair
@@ -659,11 +669,12 @@ __device__ __forceinline__ void SumSegment(const DevBatch& batch, uint32_t si, d
 
 template <int NT>
 __device__ __forceinline__ void FinishSegment(const DevBatch& batch, uint32_t si,
-                                              double* scratch) {
+                                              double* scratch, uint32_t written = 1u) {
     volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(scratch + 6 * (NT / 32));
     if (threadIdx.x == 0) {
-        __threadfence();  // this CTA's partial, before the count that publishes it
-        flag[0] = atomicAdd(&batch.seg_done[si], 1u) + 1u == __ldg(&batch.seg[si].partials);
+        __threadfence();  // this CTA's partials, before the count that publishes them
+        flag[0] = atomicAdd(&batch.seg_done[si], written) + written ==
+                  __ldg(&batch.seg[si].partials);
     }
     __syncthreads();
     if (flag[0]) SumSegment<NT>(batch, si, scratch);
@@ -754,13 +765,16 @@ __global__ void __launch_bounds__(NT, MB) Ss2BlurPersistentKernel(DevBatch batch
 // instructions as in the one-tile kernel, so they are bit-identical to it.
 // Each thread keeps its six FP32 sums across the strip's tiles (at most
 // 4 S map values per lane) and the CTA reduces them once, with two-sum
-// compensation, into one partial for the strip: the compensated reduction,
+// compensation, into one partial for the strip (float planes): the compensated reduction,
 // its barriers and its scalar adds run once per strip instead of once per
 // tile. The partial's grouping differs from one tile per CTA, so results
 // agree with that kernel to rounding (~1e-7 relative), not bit for bit.
+// Half planes keep one partial per tile, whatever the strip: their results
+// are the one-tile kernel's bits, alone and in any list.
 //
 // The reduction's scratch is rows 12..TH-1 of the horizontal planes, free
-// once the last tile's vertical pass is done.
+// between a tile's vertical pass and the next one's horizontal pass (which
+// needs only the halo moved to rows 0..11).
 template <int TW, int TH, int NT>
 struct HqScratch {
     using T = Tile<TW, TH, NT>;
@@ -809,10 +823,12 @@ __device__ __forceinline__ void RunStrip(const DevBatch& batch, uint32_t block, 
         IssueTileLoads<TW, TH, NT>(src, t);
         CpAsyncCommit();
     }
+    const HqScratch<TW, TH, NT> red{hq};
     float2 sum[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) sum[i] = make_float2(0.0f, 0.0f);
     for (int k = 0; k < count; ++k) {
+        if (kHalf || k == 0)
+#pragma unroll
+            for (int i = 0; i < 6; ++i) sum[i] = make_float2(0.0f, 0.0f);
         if constexpr (!kHalf) CpAsyncWait<0>();
         __syncthreads();
         HorizontalPass<TW, TH, NT>(batch.taps2, src, hq, k == 0 ? 0 : kRadius);
@@ -822,23 +838,33 @@ __device__ __forceinline__ void RunStrip(const DevBatch& batch, uint32_t block, 
         else
             VerticalMaps<TW, TH, NT, true>(batch.taps2, src, hq, t, sum);
         __syncthreads();  // every read of the window and of `hq` is done
-        if (k + 1 < count) {
-            t.y0 += TH;
-            if constexpr (kHalf) {
+        const bool more = k + 1 < count;
+        if (more) t.y0 += TH;
+        if constexpr (kHalf) {
+            StoreSums<NT>(sum, red);
+            if (more) {
                 HalfChunks<TW, TH, NT> chunks;
                 chunks.Load(t, kRadius / 2);
                 MoveHalo<TW, TH, NT>(hq);
                 chunks.Store(src, kRadius / 2);
-            } else {
-                IssueTileLoads<TW, TH, NT>(src, t, kRadius / 2);
-                CpAsyncCommit();
-                MoveHalo<TW, TH, NT>(hq);
             }
+            __syncthreads();
+            // (The next pass over `hq` starts behind another barrier.)
+            FoldSums<NT>(red, batch.partials + static_cast<size_t>(t.partial) * 6);
+            t.partial += seg.tiles_x;
+        } else if (more) {
+            IssueTileLoads<TW, TH, NT>(src, t, kRadius / 2);
+            CpAsyncCommit();
+            MoveHalo<TW, TH, NT>(hq);
         }
     }
-    ReducePartials<NT>(sum, HqScratch<TW, TH, NT>{hq},
-                       batch.partials + (static_cast<size_t>(seg.partial_first) + strip) * 6);
-    FinishSegment<NT>(batch, si, reinterpret_cast<double*>(src));
+    if constexpr (kHalf)
+        __syncthreads();
+    else
+        ReducePartials<NT>(
+            sum, red, batch.partials + (static_cast<size_t>(seg.partial_first) + strip) * 6);
+    FinishSegment<NT>(batch, si, reinterpret_cast<double*>(src),
+                      kHalf ? static_cast<uint32_t>(count) : 1u);
 }
 
 template <int TW, int TH, int NT, int MB, int S, bool kHalf = false>

@@ -131,7 +131,8 @@ struct DevSegment {
     uint32_t tiles_x;
     uint32_t tiles;
     uint32_t partial_first;  // index of this segment's first partial
-    uint32_t partials;       // partials the blur writes: one per CTA (a tile, or a strip)
+    uint32_t partials;       // partials the blur writes: one per CTA (a tile, or a strip),
+                             // with half planes always one per tile
 };
 
 // One image of one pair for the prepare stage. Images decoded through the

@@ -239,9 +239,11 @@ struct Tables {
     size_t partials = 0;  // tile partial count
 };
 
-// Lays out pairs of the given sizes. Plane pointers are filled later, once
-// the pyramid allocation is known (FillPointers).
-Tables BuildTables(const std::vector<std::pair<uint32_t, uint32_t>>& sizes, BlurShape shape) {
+// Lays out pairs of the given sizes, with float planes or `half` ones (whose
+// blur writes a partial per tile instead of one per CTA). Plane pointers are
+// filled later, once the pyramid allocation is known (FillPointers).
+Tables BuildTables(const std::vector<std::pair<uint32_t, uint32_t>>& sizes, BlurShape shape,
+                   bool half) {
     Tables t;
     t.pairs.resize(sizes.size());
     t.blur_start.push_back(0);
@@ -282,9 +284,10 @@ Tables BuildTables(const std::vector<std::pair<uint32_t, uint32_t>>& sizes, Blur
                 const uint32_t ty = (plan.h[l] + shape.h - 1) / shape.h;
                 s.tiles = s.tiles_x * ty;
                 s.partial_first = static_cast<uint32_t>(t.partials);
-                s.partials = BlurBlocks(shape.variant, s.tiles_x, ty);
+                const uint32_t ctas = BlurBlocks(shape.variant, s.tiles_x, ty);
+                s.partials = half ? s.tiles : ctas;
                 t.partials += s.partials;
-                blur += s.partials;
+                blur += ctas;
                 t.segs.push_back(s);
                 t.blur_start.push_back(static_cast<uint32_t>(blur));
             }
@@ -620,7 +623,7 @@ public:
         VQM_CK(cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming));
         shape_ = BlurShape::Of(
             AutoBlurVariant(DefaultTileGrids({{cfg.width, cfg.height}}), DeviceSms(device_)));
-        tables_ = BuildTables({{cfg.width, cfg.height}}, shape_);
+        tables_ = BuildTables({{cfg.width, cfg.height}}, shape_, cfg.half_planes != 0);
         BuildPrepLists(tables_, {{0, 0}});
         mem_.Layout(tables_);
         mem_.Stage(tables_);
@@ -1192,7 +1195,7 @@ public:
     size_t DeviceBytesAfter(uint32_t n, const vqm_cu_image* o, const vqm_cu_image* d) {
         std::vector<std::pair<uint32_t, uint32_t>> sizes;
         const size_t host_bytes = ValidatePairs(n, o, d, sizes);
-        Tables t = BuildTables(sizes, ShapeFor(sizes));
+        Tables t = BuildTables(sizes, ShapeFor(sizes), cfg_.half_planes != 0);
         BatchMemory probe;  // offsets only; the sizes come from mem_
         probe.elem_bytes = mem_.elem_bytes;
         const std::array<size_t, 5> need = probe.Needs(t);
@@ -1223,7 +1226,7 @@ public:
         const size_t host_bytes = ValidatePairs(n, o, d, sizes);
         VQM_CK(cudaSetDevice(device_));
         const BlurShape shape = ShapeFor(sizes);
-        Tables t = BuildTables(sizes, shape);
+        Tables t = BuildTables(sizes, shape, cfg_.half_planes != 0);
         mem_.Layout(t);
         inputs_.ensure(std::max<size_t>(host_bytes, 256));
         size_t cursor = 0;
