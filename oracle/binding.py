@@ -218,17 +218,17 @@ def source_desc(fmt: Format, chroma_filter: int = 0) -> np.ndarray:
     return words
 
 
-def pyramid(image: Image, background: float = 0.5, chroma_filter: int = 0):
-    """The FP32 XYB pyramid: list of arrays [3, H_l, W_l] (pruned = NaN)."""
+def pyramid(image: Image, background: float = 0.5, chroma_filter: int = 0, precision: int = 32):
+    """The FP32 XYB pyramid: list of arrays [3, H_l, W_l] (pruned = NaN);
+    precision 16: the half-plane build's."""
     count = ctypes.c_size_t()
     img = image.c()
-    _check(lib().ss2o_pyramid(ctypes.byref(img), ctypes.c_float(background),
-                              chroma_filter, None, 0, ctypes.byref(count)))
+    count.value = sum(3 * w * h for w, h in plan_scales(image.width, image.height))
     out = np.zeros(count.value, dtype=np.float32)
-    _check(lib().ss2o_pyramid(ctypes.byref(img), ctypes.c_float(background),
-                              chroma_filter,
-                              out.ctypes.data_as(ctypes.c_void_p), out.size,
-                              ctypes.byref(count)))
+    _check(lib().ss2o_pyramid_of(ctypes.byref(img), ctypes.c_float(background),
+                                 chroma_filter, precision,
+                                 out.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(out.size),
+                                 ctypes.byref(count)))
     levels, at = [], 0
     for (w, h) in plan_scales(image.width, image.height):
         n = 3 * w * h

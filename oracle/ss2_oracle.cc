@@ -1669,11 +1669,16 @@ int ss2o_source_desc(const ss2o_format* format, int chroma_filter,
 
 int ss2o_pyramid(const ss2o_image* image, float background, int chroma_filter,
                  float* out, size_t capacity, size_t* count) {
+    return ss2o_pyramid_of(image, background, chroma_filter, 32, out, capacity, count);
+}
+
+int ss2o_pyramid_of(const ss2o_image* image, float background, int chroma_filter,
+                    int precision, float* out, size_t capacity, size_t* count) {
     try {
         const Plan plan = PlanScales(image->width, image->height);
         const Desc d = BuildDesc(image->format, chroma_filter);
         Pyramid<float> p;
-        BuildPyramid<float>(*image, d, background, plan, p);
+        BuildPyramid<float>(*image, d, background, plan, p, precision == 16);
         size_t total = 0;
         for (int l = 0; l < plan.count; ++l)
             total += size_t(3) * plan.sizes[l].w * plan.sizes[l].h;

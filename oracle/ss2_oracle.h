@@ -106,6 +106,9 @@ int ss2o_source_desc(const ss2o_format* format, int chroma_filter,
  * level. Returns the float count through *count. */
 int ss2o_pyramid(const ss2o_image* image, float background, int chroma_filter,
                  float* out, size_t capacity, size_t* count);
+/* The same at precision 32, or 16: the half-plane build's planes. */
+int ss2o_pyramid_of(const ss2o_image* image, float background, int chroma_filter,
+                    int precision, float* out, size_t capacity, size_t* count);
 /* Raw per-level norm sums (18 floats per level) of the FP32 path. */
 int ss2o_level_sums(const ss2o_image* original, const ss2o_image* distorted,
                     float background, int chroma_filter, float* sums,

@@ -37,6 +37,12 @@ FORMATS = {
     "pq420p10_center": _hdr(T.St2084, chroma_location=ss2.ChromaLocation.Center),
     "hlg422p10": _hdr(T.AribB67, subsample_h=0),
     "hlg420p8": _hdr(T.AribB67, type=ss2.PixelType.Byte, depth=0),
+    # No primaries matrix behind the transfer: its last product is the linear
+    # value that the box sums and the opsin mix read.
+    "pq420p10_bt709": _hdr(T.St2084, primaries=ss2.ColorPrimaries.Bt709),
+    "hlg420p10_bt709": _hdr(T.AribB67, primaries=ss2.ColorPrimaries.Bt709),
+    "pq_grey16": F(type=ss2.PixelType.Word, family=ss2.ColorFamily.Grey, matrix=M.Bt709,
+                   transfer=T.St2084),
     "pq444p12": _hdr(T.St2084, depth=12, subsample_w=0, subsample_h=0),
     "ictcp_pq420p10": _hdr(T.St2084, matrix=M.Bt2100ICtCp),
     "srgb_yuv420p8": _hdr(T.Srgb, type=ss2.PixelType.Byte, depth=0, matrix=M.Bt709,
@@ -48,6 +54,8 @@ FORMATS = {
     "grey16": F(type=ss2.PixelType.Word, family=ss2.ColorFamily.Grey, matrix=M.Bt709),
     "rgb_float": F(),
     "rgb_half_linear": F(type=ss2.PixelType.Half, transfer=T.Linear),
+    "hlg_float_bt709": _hdr(T.AribB67, type=ss2.PixelType.Float, depth=0, subsample_w=0,
+                            subsample_h=0, primaries=ss2.ColorPrimaries.Bt709),
     "pq_float": _hdr(T.St2084, type=ss2.PixelType.Float, depth=0, subsample_w=0, subsample_h=0),
 }
 
@@ -69,11 +77,11 @@ def _image(fmt, w, h, seed, wild):
     return img
 
 
-def _check_planes(pipe, images, w, h):
+def _check_planes(pipe, images, w, h, precision=32):
     from oracle import binding as ob
     scales = len(ss2.plan_scales(w, h))
     for image, img in enumerate(images):
-        want = ob.pyramid(helpers.to_oracle(img), 0.3)
+        want = ob.pyramid(helpers.to_oracle(img), 0.3, precision=precision)
         for level in range(scales):
             for c in range(3):
                 if not ob.channel_pruned(c, level, scales):
@@ -98,6 +106,52 @@ def test_planes_bit_exact(name, wild):
         with ss2.Ssimulacra2Pipeline(w, h) as p:
             p.compute(*images, 0.3)
             _check_planes(p, images, w, h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(FORMATS))
+def test_half_planes_bit_exact(name):
+    """The binary16 stores, averages and padding blocks of the curve kernel."""
+    fmt = FORMATS[name]
+    sizes = [(200, 134), (66, 130)] if fmt.subsample_w else [(201, 133), (67, 65)]
+    for w, h in sizes:
+        images = [_image(fmt, w, h, s, False) for s in (3, 4)]
+        with ss2.Ssimulacra2Pipeline(w, h, half_planes=True) as p:
+            p.compute(*images, 0.3)
+            _check_planes(p, images, w, h, precision=16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("name,w,h", [("pq420p10", 1664, 1472), ("rgb16", 1663, 1471)])
+def test_large_single_pair_bit_exact(name, w, h, half):
+    """One pair of 1,196 tiles, more than two waves (1,184): the one-pair
+    kernel of 128 threads, as a graph's first launch and its next replay."""
+    fmt = FORMATS[name]
+    images = [_image(fmt, w, h, s, False) for s in (6, 7)]
+    with ss2.Ssimulacra2Pipeline(w, h, half_planes=half) as p:
+        p.compute(images[1], images[0], 0.3)
+        p.compute(*images, 0.3)
+        _check_planes(p, images, w, h, precision=16 if half else 32)
+
+
+@pytest.mark.gpu
+def test_one_pair_replays_with_two_decodes():
+    """Images of different decode groups give a captured call two prepare
+    launches; each replay takes its own pair's record in both."""
+    w, h = 258, 130
+    names = [("pq420p10", "rgb8"), ("rgb8", "pq420p10"), ("rgba8", "yuv"), ("yuv", "rgb8"),
+             ("pq420p10", "hlg422p10")]
+    formats = dict(FORMATS, rgb8=F(type=ss2.PixelType.Byte),
+                   yuv=_hdr(T.Bt709, matrix=M.Bt709, primaries=ss2.ColorPrimaries.Bt709))
+    pairs = [tuple(_image(formats[n], w, h, 10 * k + i, False) for i, n in enumerate(pair))
+             for pair in names for k in range(2)]
+    with ss2.Ssimulacra2Pipeline(w, h) as p, ss2.Ssimulacra2Pipeline(w, h) as plain:
+        plain.set_graphs(False)
+        for images in pairs + pairs[::-1]:
+            got = p.compute(*images, 0.3)
+            _check_planes(p, images, w, h)
+            assert np.array_equal(got.norms, plain.compute(*images, 0.3).norms)
 
 
 @pytest.mark.gpu
