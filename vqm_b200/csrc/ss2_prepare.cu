@@ -178,7 +178,7 @@ __device__ __forceinline__ float BoxAverage(float a, float b, float c, float d) 
 struct LevelInfo {
     void* plane[kMaxLevels][3];  // nullptr when pruned
     uint32_t w[kMaxLevels], h[kMaxLevels], pitch[kMaxLevels], mask[kMaxLevels];
-    uint32_t levels;
+    uint32_t last;  // the deepest level that stores a channel
 };
 
 template <bool kHalf>
@@ -418,7 +418,14 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
             lv.mask[tid] = tid < P.levels ? P.mask[tid] : 0u;
         }
         if (tid == 0) {
-            lv.levels = P.levels;
+            // (Read from here where it is needed, and no block counts beside
+            // the sizes: the table kernels' 48 registers spill 28-36 bytes so,
+            // 60-80 with each thread's own search, and the table prepare of
+            // 64 1080p pairs takes 1033 us instead of 1040.)
+            uint32_t last = 0;
+            for (uint32_t l = 1; l < P.levels; ++l)
+                if (P.mask[l]) last = l;
+            lv.last = last;
             // 32-bit sample loads need every plane and row on a 4-byte boundary.
             const DevSource& ps = P.src[image];
             uint32_t ok = 1;
@@ -445,17 +452,11 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
             __syncthreads();
         }
     }
-    const uint32_t levels = lv.levels;
     const uint32_t width = s.width, height = s.height;
-    const uint32_t wb = (width + 1) / 2, hb = (height + 1) / 2;  // base blocks
     // Blocks of level 0's plane, padding included (ss2_layout.h).
     const uint32_t wb_pad = PaddedColumns(width, kHalf) / 2;
     const uint32_t tx = tid & 15, ty = tid >> 4;
     const uint32_t mask0 = lv.mask[0];
-
-    uint32_t last = 0;  // the deepest level that stores a channel
-    for (uint32_t l = 1; l < levels; ++l)
-        if (lv.mask[l]) last = l;
 
 #pragma unroll 1
     for (uint32_t vy = 0; vy < kRowPasses; ++vy) {
@@ -488,8 +489,8 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
         for (uint32_t hx = 0; hx < 2; ++hx) {
             const uint32_t bx = bx0 + hx;
             float lin[4][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-            const bool in_block = bx < wb && by < hb;
-            if (kHalf && !in_block && bx < wb_pad && by < hb && mask0) {
+            const bool in_block = 2 * bx < width && 2 * by < height;
+            if (kHalf && !in_block && bx < wb_pad && 2 * by < height && mask0) {
                 // Padding blocks past the image's last column: zeros.
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
@@ -546,7 +547,7 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
             }
         }
         // Level 1: pixels (bx0, by) and (bx0 + 1, by).
-        if (last >= 1) {
+        if (lv.last >= 1) {
             float2 xyb[3];
             Xyb2<kInRange>(make_float2(l1[0][0], l1[1][0]), make_float2(l1[0][1], l1[1][1]),
                            make_float2(l1[0][2], l1[1][2]), lv.mask[1], xyb);
@@ -571,7 +572,7 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
                 StorePixel<kHalf>(lv, 1, bx0, by, xyb[0].x, xyb[1].x, xyb[2].x);
                 StorePixel<kHalf>(lv, 1, bx0 + 1, by, xyb[0].y, xyb[1].y, xyb[2].y);
             }
-            if (last >= 2) {
+            if (lv.last >= 2) {
                 const uint32_t at = (ty + kRows * vy) * kBlocks + 2 * tx;  // even
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
@@ -579,7 +580,7 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
             }
         }
     }
-    if (last < 2) return;
+    if (lv.last < 2) return;
     __syncthreads();
 
     // Levels 2..last: the first side^2 / 2 threads average the previous
@@ -590,9 +591,9 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
     // repeats it (the clamp to its last column and row); a pixel past the
     // level is averaged from zeros and not stored. Threads that no longer
     // take part leave, and the rest meet at a barrier of their own. (One
-    // pixel a thread: table prepare of 64 1080p pairs 1.149 ms, now 1.042.)
+    // pixel at a time: table prepare of 64 1080p pairs 1.084 ms, now 1.033.)
 #pragma unroll 1
-    for (uint32_t level = 2; level <= last; ++level) {
+    for (uint32_t level = 2; level <= lv.last; ++level) {
         const uint32_t shift = 5 - level;             // side / 2 = 32 >> level
         const uint32_t side = 2u << shift;
         const uint32_t workers = side << shift;       // side^2 / 2, at most 128
@@ -621,7 +622,7 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
         const uint32_t x = gx * side + jx, y = gy * side + jy;
         StorePixel<kHalf>(lv, level, x, y, xyb[0].x, xyb[1].x, xyb[2].x);
         StorePixel<kHalf>(lv, level, x + 1, y, xyb[0].y, xyb[1].y, xyb[2].y);
-        if (level < last) {
+        if (level < lv.last) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
                 *reinterpret_cast<float2*>(next0 + c * next_stride + jy * side + jx) = v[c];
