@@ -47,6 +47,9 @@ FORMATS = {
     "ictcp_pq420p10": _hdr(T.St2084, matrix=M.Bt2100ICtCp),
     "srgb_yuv420p8": _hdr(T.Srgb, type=ss2.PixelType.Byte, depth=0, matrix=M.Bt709,
                           primaries=ss2.ColorPrimaries.Bt709),
+    # The BT.2020 matrix's inverse has entries of 2^-56 for 0, so the device
+    # tests this image's values for tiny ones.
+    "srgb_yuv420p16_bt2020": _hdr(T.Srgb, depth=0, range=ss2.PixelRange.Full),
     "rgb16": F(type=ss2.PixelType.Word),
     "rgb10": F(type=ss2.PixelType.Word, depth=10),
     "rgba8": F(type=ss2.PixelType.Byte, alpha=ss2.AlphaType.Straight),

@@ -739,11 +739,14 @@ __device__ __forceinline__ float2 CurvePow2(float2 x, float y, const CurveTables
     return make_float2(CurvePow(x.x, y, tab), CurvePow(x.y, y, tab));
 }
 
-// TransferDecode's curves for two pixels whose values are 0 or at least 2^-100
-// and below 12 in magnitude (HLG's exponential overflows a float at 16.4).
+// TransferDecode's curves for two pixels whose values are below 12 in magnitude
+// (HLG's exponential overflows a float at 16.4) and, for sRGB, 0 or at least
+// 2^-100.
 //
 // St2084Eotf. (Its scalar subtractions: a two-lane product feeding a two-lane
-// sum comes out as one fused operation.)
+// sum comes out as one fused operation.) Below 2^-21 the difference n is
+// negative and the value 0, whatever CurvePow makes of a subnormal x (less
+// than 1/2).
 __device__ __forceinline__ float2 CurveSt2084(float2 x, const CurveTables& tab) {
     const bool la = x.x > 0.0f, lb = x.y > 0.0f;
     const float2 xp = CurvePow2(make_float2(la ? x.x : 1.0f, lb ? x.y : 1.0f), 1.0f / 78.84375f,

@@ -88,11 +88,11 @@ struct DevSourceHead {
     // parity, so the host fixes the first window slot and the four tap
     // weights per parity. Also requires the YUV matrix to map every sample
     // code below the transfer power's fast-range limit.
-    // The curve path (BlockLinearCurve): any sample type and family, alpha
-    // included, whose transfer is linear, sRGB, ST 2084 or HLG, outside the
-    // constant-luminance mode; its subsampled chroma, if any, is integer,
-    // bilinear and by at most 2, with the phases below. 2: no value the
-    // transfer meets is tiny (CurveRgb); 1: it looks.
+    // The curve path (CurveRow, ss2_decode.cuh): any sample type and family,
+    // alpha included, whose transfer is linear, sRGB, ST 2084 or HLG, outside
+    // the constant-luminance mode; its subsampled chroma, if any, is integer,
+    // bilinear and by at most 2, with the phases below. 1: an sRGB image whose
+    // values CurveRgb tests for tiny ones; 2: it need not.
     uint8_t yuv_fast;
     uint8_t curve;
     uint8_t chroma_pattern;    // 4:2:0 phases known at compile time: 1 + x type

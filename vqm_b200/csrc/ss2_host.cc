@@ -502,6 +502,53 @@ bool ChromaPhases(const vqm_cu_format& f, DevSource& d) {
     return true;
 }
 
+// The exponent of the largest power of two that v is a multiple of (0: of
+// any; not finite: of none).
+int Grain(float v) {
+    uint32_t bits;
+    std::memcpy(&bits, &v, 4);
+    const int field = static_cast<int>(bits >> 23 & 255u);
+    uint32_t m = (bits & 0x7fffffu) | (field ? 0x800000u : 0u);
+    if (field == 255) return -100000;
+    if (m == 0) return 100000;
+    int e = std::max(field, 1) - 150;
+    for (; !(m & 1u); m >>= 1) ++e;
+    return e;
+}
+
+// Whether every value an sRGB image's transfer meets is 0 or at least 2^-100
+// in magnitude (the range of the device's division by 12.92). Integer samples
+// enter as codes times a scale plus an offset, and every step after that adds
+// products: with the factors' Grain known, so is a power of two that every
+// intermediate value is a multiple of, which rounding to a float keeps, so
+// that a value is 0 or at least that power. Premultiplied alpha divides, and
+// float samples have no grain.
+bool SrgbValuesNotTiny(const vqm_cu_format& f, const DevSource& d) {
+    if (f.type > 1 || f.alpha == 2) return false;
+    int code[3];  // luma, chroma, alpha samples
+    for (int i = 0; i < 3; ++i) code[i] = std::min(Grain(d.scale[i]), Grain(d.offset[i]));
+    int q[3] = {code[0], code[0], code[0]};
+    if (f.family == 2) {
+        int weight = d.chroma_variant ? 100000 : 0;
+        if (d.chroma_variant)
+            for (int i = 0; i < 16; ++i)
+                weight = std::min(weight, Grain(d.cweight[i >> 3][(i >> 2) & 1][i & 3]));
+        q[1] = q[2] = code[1] + weight;
+    }
+    int least = 100000;
+    for (int row = 0; row < 3; ++row) {
+        int g = q[row];
+        if (!d.identity1) {
+            g = 100000;
+            for (int j = 0; j < 3; ++j) g = std::min(g, Grain(d.m1[3 * row + j]) + q[j]);
+        }
+        if (f.alpha == 1)  // alpha * value + (1 - alpha) * background
+            g = std::min(code[2] + g, std::min(code[2], 0) + Grain(d.background));
+        least = std::min(least, g);
+    }
+    return least >= -100;
+}
+
 // The decode paths with a chroma window of their own: sets yuv_fast and
 // gamma, curve, and the chroma phases both use. Returns a bound on the
 // magnitude of the YUV matrix's outputs over every sample code for the YUV
@@ -521,15 +568,11 @@ double FastDecodeConstants(const vqm_cu_format& f, int mode, int tid, uint32_t c
     const bool window = f.family == 2 && f.type <= 1 && f.subsample_w <= 1 &&
                         f.subsample_h <= 1 && (!d.chroma_variant || chroma_filter == 0) &&
                         ChromaPhases(f, d);
-    d.curve = curve && (window || !d.chroma_variant) ? 1 : 0;
-    // Integer samples' values are 0 or above 2^-100: a code times its scale
-    // plus the offset is a multiple of 2^-40, alpha is 0 or above 2^-17, and
-    // the matrix entries are 0 or above 2^-58 (0 can come out of the inversion
-    // as about 2^-55).
-    const float bg = std::fabs(d.background);
-    if (d.curve && f.type <= 1 &&
-        (f.alpha == 0 || (f.alpha == 1 && (bg == 0.0f || (bg >= 1e-6f && bg <= 4.0f)))))
-        d.curve = 2;
+    // Only sRGB's linear part divides a value that can be tiny: ST 2084 maps
+    // everything below 2^-21 to 0 and HLG squares.
+    d.curve = !curve || (d.chroma_variant && !window) ? 0
+              : tid == 4 && !SrgbValuesNotTiny(f, d)  ? 1
+                                                      : 2;
     if (!(power && window && f.alpha == 0 && mode == 0)) return none;
     const float gammas[4] = {0.0f, 2.4f, 2.2f, 2.8f};  // TransferDecode cases 1-3
     d.gamma = gammas[tid];
