@@ -17,9 +17,8 @@ from __future__ import annotations
 
 import collections
 import ctypes
-import functools
 import os
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Iterable, Sequence
 
 import numpy as np
@@ -450,12 +449,29 @@ class Ssimulacra2Scale:
 class Ssimulacra2Result:
     norms: np.ndarray  # [scales, 18]
     device_score: float | None = None
+    scales: list = field(init=False)
 
-    # Made when first read: building the scales of 64 results took 0.4 ms of a
-    # 3.4 ms list of 1080p pairs, which reads none of them.
-    @functools.cached_property
-    def scales(self) -> list:
-        return [Ssimulacra2Scale(r[:6].copy(), r[6:].copy()) for r in self.norms]
+    # The scales are those of the norms as made. Where these are the usual
+    # array, their bytes are kept and the scales built when first read: doing
+    # that for 64 results took 0.4 ms of a 3.4 ms list of 1080p pairs, which
+    # reads none.
+    def __post_init__(self):
+        n = self.norms
+        if type(n) is np.ndarray and n.ndim == 2 and n.dtype.char == "d":
+            self._made = n.tobytes(), n.shape
+        else:
+            self.scales = self._scales_of(n)
+
+    @staticmethod
+    def _scales_of(norms) -> list:
+        return [Ssimulacra2Scale(r[:6].copy(), r[6:].copy()) for r in norms]
+
+    def __getattr__(self, name):
+        made = self.__dict__.get("_made") if name == "scales" else None
+        if made is None:
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        self.scales = self._scales_of(np.frombuffer(made[0]).reshape(made[1]))
+        return self.scales
 
     def score(self) -> float:
         """Ssimulacra2Result::Score (score.cc:118-163), FP64 on the host."""
@@ -881,13 +897,13 @@ class Ssimulacra2Batch:
                                               scales.ctypes.data, scores.ctypes.data)
         self._borrowed = None
         _check(status)
-        # Each result's norms are its rows of the call's one array.
+        # (A copy each: a kept result does not keep the list's array.)
         ks = scales.tolist()
         if all(k == 6 for k in ks):
             rows = norms.reshape(n, 6, 18)
         else:
             rows = [norms[i, : 18 * k].reshape(k, 18) for i, k in enumerate(ks)]
-        return [Ssimulacra2Result(r, s) for r, s in zip(rows, scores.tolist())]
+        return [Ssimulacra2Result(r.copy(), s) for r, s in zip(rows, scores.tolist())]
 
     def compute_many(self, pairs, background: float = 0.5):
         return self.finish(self.submit(pairs, background))
