@@ -367,14 +367,18 @@ int vqm_cu_ss2_check_division(uint32_t first_bits, uint32_t last_bits,
 /* Which device decode an image of format `format` takes (a diagnostic; no
  * device is touched): VQM_CU_DECODE_GENERIC, _TABLE (8-bit grey/RGB through a
  * per-image table), _TABLE_IN_RANGE (the same, with every linear sample
- * non-negative so the cube roots need no range check) or _YUV (integer YUV
+ * non-negative so the cube roots need no range check), _YUV (integer YUV
  * with a power-law transfer and at most 2x chroma subsampling, phases fixed
- * per pixel parity; an image of such a format with an odd width or height
- * runs the generic decode). The results are the same whichever path runs. */
+ * per pixel parity) or _CURVE (any other image whose transfer is linear, sRGB,
+ * ST 2084 or HLG, with its chroma at full resolution or integer, bilinear and
+ * subsampled by at most 2x). An image of a YUV format with an odd width or
+ * height runs the generic decode in place of _YUV, and of _CURVE where its
+ * chroma is subsampled. The results are the same whichever path runs. */
 #define VQM_CU_DECODE_GENERIC 0
 #define VQM_CU_DECODE_TABLE 1
 #define VQM_CU_DECODE_TABLE_IN_RANGE 2
 #define VQM_CU_DECODE_YUV 3
+#define VQM_CU_DECODE_CURVE 4
 int vqm_cu_ss2_decode_path(const vqm_cu_format* format, uint32_t chroma_filter,
                            uint32_t* path);
 

@@ -101,6 +101,7 @@ def _check_planes(pipe, images, w, h, precision=32):
 @pytest.mark.parametrize("name", list(FORMATS))
 def test_planes_bit_exact(name, wild):
     fmt = FORMATS[name]
+    assert ss2.decode_path(fmt) == "curve"
     sizes = [(200, 134), (66, 130)]
     if not fmt.subsample_w:
         sizes += [(201, 133), (67, 65)]

@@ -24,8 +24,8 @@ def _yuv(**kw):
        matrix=ss2.MatrixCoefficients.Bt709), 0, "table_in_range"),
     (F(type=ss2.PixelType.Byte, range=ss2.PixelRange.Limited), 0, "table"),
     (F(type=ss2.PixelType.Byte, primaries=ss2.ColorPrimaries.Bt2020), 0, "table"),
-    (F(type=ss2.PixelType.Byte, alpha=ss2.AlphaType.Straight), 0, "generic"),
-    (F(type=ss2.PixelType.Float), 0, "generic"),
+    (F(type=ss2.PixelType.Byte, alpha=ss2.AlphaType.Straight), 0, "curve"),
+    (F(type=ss2.PixelType.Float), 0, "curve"),
     (_yuv(), 0, "yuv"),
     (_yuv(chroma_location=ss2.ChromaLocation.Center), 0, "yuv"),
     (_yuv(chroma_location=ss2.ChromaLocation.TopLeft), 0, "yuv"),
@@ -38,8 +38,13 @@ def _yuv(**kw):
     (_yuv(primaries=ss2.ColorPrimaries.Bt2020, matrix=ss2.MatrixCoefficients.Bt2020Ncl,
           transfer=T.Bt2020_10), 0, "yuv"),
     (_yuv(), 1, "generic"),                       # bicubic chroma
-    (_yuv(transfer=T.Srgb), 0, "generic"),         # not a pure power law
-    (_yuv(transfer=T.St2084), 0, "generic"),
+    (_yuv(transfer=T.Srgb), 0, "curve"),           # not a pure power law
+    (_yuv(transfer=T.St2084), 0, "curve"),
+    (_yuv(transfer=T.AribB67, type=ss2.PixelType.Float, depth=0, subsample_w=0, subsample_h=0), 0,
+     "curve"),
+    (_yuv(transfer=T.St2084), 1, "generic"),       # bicubic chroma
+    (_yuv(transfer=T.St2084, type=ss2.PixelType.Float, depth=0), 0, "generic"),
+    (_yuv(transfer=T.Log100), 0, "generic"),
     (_yuv(subsample_w=2, subsample_h=0), 0, "generic"),  # 4:1:1
     (_yuv(alpha=ss2.AlphaType.Straight), 0, "generic"),
     (_yuv(type=ss2.PixelType.Float, depth=0), 0, "generic"),

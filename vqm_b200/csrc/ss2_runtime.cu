@@ -1450,7 +1450,7 @@ struct vqm_cu_ss2_batch {
 extern "C" {
 
 const char* vqm_cu_last_error(void) { return vqm_b200::g_last_error.c_str(); }
-uint32_t vqm_cu_version(void) { return (1u << 16) | 5u; }
+uint32_t vqm_cu_version(void) { return (1u << 16) | 6u; }
 
 int vqm_cu_device_count(uint32_t* count) {
     return vqm_b200::Guard([&] {
@@ -1859,7 +1859,9 @@ int vqm_cu_ss2_decode_path(const vqm_cu_format* format, uint32_t chroma_filter,
         vqm_b200::DevSource d{};
         vqm_b200::BuildSourceConstants(*format, chroma_filter, 0.5f, d);
         *path = d.lut ? (d.in_range ? VQM_CU_DECODE_TABLE_IN_RANGE : VQM_CU_DECODE_TABLE)
-                      : (d.yuv_fast ? VQM_CU_DECODE_YUV : VQM_CU_DECODE_GENERIC);
+                : d.yuv_fast ? VQM_CU_DECODE_YUV
+                : d.curve    ? VQM_CU_DECODE_CURVE
+                             : VQM_CU_DECODE_GENERIC;
     });
 }
 

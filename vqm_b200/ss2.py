@@ -771,16 +771,18 @@ class Ssimulacra2Pipeline:
 
 VARIANT_WORDS = 5
 
-DECODE_PATHS = ("generic", "table", "table_in_range", "yuv")
+DECODE_PATHS = ("generic", "table", "table_in_range", "yuv", "curve")
 
 
 def decode_path(fmt: "ImageFormat", chroma_filter: int = 0) -> str:
     """Which device decode images of `fmt` take (the results are the same
     whichever runs): "generic", "table" (8-bit grey/RGB through a table),
-    "table_in_range" (the same, non-negative linear samples) or "yuv"
-    (integer YUV, power-law transfer, at most 2x chroma subsampling; an
-    image of such a format with an odd width or height runs the generic
-    decode)."""
+    "table_in_range" (the same, non-negative linear samples), "yuv"
+    (integer YUV, power-law transfer, at most 2x chroma subsampling) or
+    "curve" (other images with a linear, sRGB, ST 2084 or HLG transfer, their
+    chroma at full resolution or integer, bilinear and at most 2x subsampled).
+    An image of a YUV format with an odd width or height runs the generic
+    decode in place of "yuv", and of "curve" where its chroma is subsampled."""
     path = ctypes.c_uint32()
     _check(_lib.vqm_cu_ss2_decode_path(ctypes.byref(fmt), chroma_filter, ctypes.byref(path)))
     return DECODE_PATHS[path.value]
