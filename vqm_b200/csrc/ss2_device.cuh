@@ -135,10 +135,9 @@ struct DevSegment {
                              // with half planes always one per tile
 };
 
-// One image of one pair for the prepare stage. Images decoded through the
-// 8-bit table come first in the list, the rest (generic decode) after them,
-// each group with its own prefix offsets, so each group is one launch of its
-// own specialised kernel.
+// One image of one pair for the prepare stage of a batch. The list is in
+// prepare groups (below), each with its own prefix offsets, so each group is
+// one launch of its own specialised kernel.
 struct DevPrepItem {
     uint32_t pair;
     uint32_t image;

@@ -242,8 +242,8 @@ void Run(const vqm_cu_image* o, const vqm_cu_image* d, float background, uint32_
     P.pyramid = reinterpret_cast<float*>(base + off_pyramid);
     P.result = result;
 
-    // Prepare lists: the two images by prepare group (table, YUV, generic),
-    // each group's prefix offsets after the previous group's.
+    // Prepare lists: the two images by prepare group (PrepGroup), each
+    // group's prefix offsets after the previous group's.
     const uint32_t per_image = P.prep_tiles_x * P.prep_tiles_y;
     const int group[2] = {PrepGroup(P.src[0]), PrepGroup(P.src[1])};
     uint32_t n[kPrepGroups] = {};

@@ -43,9 +43,9 @@ namespace {
 constexpr uint32_t kBlocks = kPrepTile / 2;  // base 2x2 blocks per tile side
 
 // CTAs per SM of a prepare kernel of 128 threads (large launches): ten for
-// the table decode, eight for the YUV decode with its 4:2:0 chroma window
-// (28 KB of shared memory); the 256-thread kernels run five or four (see
-// PrepareKernel).
+// the table decode, eight for the YUV and curve decodes with their 4:2:0
+// chroma window (28 KB of shared memory); the 256-thread kernels run five or
+// four (see kPrepareCtas).
 constexpr int kTableCtas128 = 10;
 constexpr int kYuvCtas128 = 8;
 // The curve decode: as many warps of 64 registers as the YUV decode (a 4K
@@ -338,8 +338,8 @@ __device__ __forceinline__ void CurveBlock(const DevSourceHead& s, const CurveWo
 }
 
 // CTAs per SM: five of 256 threads (40 warps) for the table and YUV
-// decodes, four for the generic one; the table decode also runs as ten CTAs
-// of 128 threads (see LaunchPrepareOf). The decodes' long dependency chains
+// decodes, four for the generic and curve ones; all but the generic one also
+// run as CTAs of 128 threads (see LaunchPrepareOf). The decodes' long dependency chains
 // (the YUV power's table loads, the generic FP64 transfers) want the warps
 // more than the registers (measured on 136 uneven pairs: the YUV kernel at
 // 5 CTAs with some spilling took 8.48 ms, at 4 9.33 ms; the generic decode
@@ -351,8 +351,11 @@ __device__ __forceinline__ void CurveBlock(const DevSourceHead& s, const CurveWo
 #ifndef VQM_YUV_PREPARE_CTAS
 #define VQM_YUV_PREPARE_CTAS 5
 #endif
+constexpr int kPrepareCtas128[kPrepGroups] = {kTableCtas128, kYuvCtas128, 0, kCurveCtas128};
+constexpr int kPrepareCtas256[kPrepGroups] = {5, VQM_YUV_PREPARE_CTAS, VQM_GENERIC_PREPARE_CTAS,
+                                              kCurveCtas256};
 template <int kGroup, int kNT>
-constexpr int kPrepareCtas = kNT == 128 ? (kGroup == 0 ? kTableCtas128 : kGroup == 3 ? kCurveCtas128 : kYuvCtas128) : kGroup == 0 ? 5 : kGroup == 1 ? VQM_YUV_PREPARE_CTAS : kGroup == 3 ? kCurveCtas256 : VQM_GENERIC_PREPARE_CTAS;
+constexpr int kPrepareCtas = kNT == 128 ? kPrepareCtas128[kGroup] : kPrepareCtas256[kGroup];
 
 // Tile t of one image of pair P.
 template <int kGroup, bool kHalf, int kNT>
@@ -371,10 +374,10 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
     __shared__ DevSourceHead src_s;  // (the byte table goes to `lut`)
     __shared__ LevelInfo lv;
     __shared__ uint32_t aligned4;
-    // Both chroma planes' window of the tile, for yuv_fast images, and the
-    // power's tables.
-    // The 128-thread YUV kernel stages 4:2:0 windows only (the host sends
-    // it launches whose images all have 4:2:0 chroma or none subsampled).
+    // Both chroma planes' window of the tile, for yuv_fast and curve images,
+    // and the powers' tables.
+    // The 128-thread kernels stage 4:2:0 windows only (the host sends them
+    // launches whose images all have 4:2:0 chroma or none subsampled).
     constexpr int kStagePlane = kNT == 128 ? kChromaStage420 : kChromaStage;
     __shared__ float chroma_stage[kYuv || kCurve ? 2 * kStagePlane : 1];
     __shared__ float pow_table[kYuv ? PowTable::kFloats : 1];
@@ -500,8 +503,8 @@ __device__ __forceinline__ void PrepareTile(const DevPair& P, int image, uint32_
             }
             if (in_block) {
                 if constexpr (kCurve) {
-                    CurveBlock<kHalf>(s, cw, chroma_stage, kStagePlane, curve_tables, gx,
-                                                gy, hx, bx, by, lv, mask0, lin);
+                    CurveBlock<kHalf>(s, cw, chroma_stage, kStagePlane, curve_tables, gx, gy, hx,
+                                      bx, by, lv, mask0, lin);
                 } else if constexpr (kTable) {
                     TableBlock(s, lut, fast, w4, hx, bx, by, lin);
                 } else if constexpr (kYuv) {

@@ -363,10 +363,9 @@ struct BatchMemory {
     DeviceBuffer table, pyramid, partials, seg_sums, pair_done;
     PinnedBuffer table_host, results_host;
     // Table layout: [pairs | prep items | prep starts | segments | blur
-    // starts]. Everything a call can change (pair records, which images take
-    // the table path) sits in the first `head_bytes`.
+    // starts].
     size_t off_pairs = 0, off_items = 0, off_prep = 0, off_segs = 0, off_blur = 0;
-    size_t head_bytes = 0, table_bytes = 0;
+    size_t table_bytes = 0;
     DevBatch dev{};
     uint32_t pair_count = 0;
     size_t elem_bytes = 4;  // pyramid element: float, or binary16 with half planes
@@ -383,8 +382,7 @@ struct BatchMemory {
         off_pairs = 0;
         off_items = AlignUp(off_pairs + sizeof(DevPair) * t.pairs.size(), 16);
         off_prep = AlignUp(off_items + sizeof(DevPrepItem) * t.prep_items.size(), 16);
-        head_bytes = AlignUp(off_prep + sizeof(uint32_t) * t.prep_start.size(), 256);
-        off_segs = head_bytes;
+        off_segs = AlignUp(off_prep + sizeof(uint32_t) * t.prep_start.size(), 256);
         off_blur = AlignUp(off_segs + sizeof(DevSegment) * t.segs.size(), 256);
         table_bytes = AlignUp(off_blur + sizeof(uint32_t) * t.blur_start.size(), 256);
         return {table_bytes, std::max<size_t>(t.pyramid_floats, 64) * elem_bytes,
@@ -442,7 +440,8 @@ struct BatchMemory {
         return moved;
     }
 
-    // Writes the host mirror of the tables with device pointers filled in.
+    // Writes the host mirror of the tables, and the kernel parameters that
+    // come from them, with device pointers filled in.
     void Stage(Tables& t) {
         for (size_t i = 0; i < t.pairs.size(); ++i) {
             t.pairs[i].pyramid =
@@ -456,12 +455,6 @@ struct BatchMemory {
         std::memcpy(h + off_pairs, t.pairs.data(), sizeof(DevPair) * t.pairs.size());
         std::memcpy(h + off_segs, t.segs.data(), sizeof(DevSegment) * t.segs.size());
         std::memcpy(h + off_blur, t.blur_start.data(), sizeof(uint32_t) * t.blur_start.size());
-        StagePrep(t);
-    }
-    // The prepare lists (after BuildPrepLists) into the host mirror and the
-    // kernel parameters.
-    void StagePrep(const Tables& t) {
-        uint8_t* h = table_host.as<uint8_t>();
         std::memcpy(h + off_items, t.prep_items.data(), sizeof(DevPrepItem) * t.prep_items.size());
         std::memcpy(h + off_prep, t.prep_start.data(), sizeof(uint32_t) * t.prep_start.size());
         for (int g = 0; g < kPrepGroups; ++g) {
@@ -473,8 +466,8 @@ struct BatchMemory {
         return reinterpret_cast<DevPair*>(table_host.as<uint8_t>() + off_pairs) + i;
     }
 
-    void EnqueueUpload(size_t bytes, cudaStream_t s) {
-        VQM_CK(cudaMemcpyAsync(table.as<void>(), table_host.as<void>(), bytes,
+    void EnqueueUpload(cudaStream_t s) {
+        VQM_CK(cudaMemcpyAsync(table.as<void>(), table_host.as<void>(), table_bytes,
                                cudaMemcpyHostToDevice, s));
     }
     // ev, when given, holds 4 timing events recorded before prepare and
@@ -624,7 +617,9 @@ public:
         shape_ = BlurShape::Of(
             AutoBlurVariant(DefaultTileGrids({{cfg.width, cfg.height}}), DeviceSms(device_)));
         tables_ = BuildTables({{cfg.width, cfg.height}}, shape_, cfg.half_planes != 0);
-        BuildPrepLists(tables_, {{0, 0}});
+        // (No prepare lists: the pair's record travels with the launch.)
+        tables_.prep_items.clear();
+        tables_.prep_start.clear();
         mem_.Layout(tables_);
         mem_.Stage(tables_);
         VQM_CK(cudaMemcpy(mem_.table.as<void>(), mem_.table_host.as<void>(), mem_.table_bytes,
@@ -1279,7 +1274,7 @@ public:
         // blur writes them into pinned host memory.
         VQM_CK(cudaMemsetAsync(mem_.pair_done.as<void>(), 0,
                                sizeof(uint32_t) * (n + t.segs.size() + 2), copy_stream_));
-        mem_.EnqueueUpload(mem_.table_bytes, copy_stream_);
+        mem_.EnqueueUpload(copy_stream_);
         VQM_CK(cudaEventRecord(uploaded_, copy_stream_));
         VQM_CK(cudaStreamWaitEvent(stream_, uploaded_, 0));
         mem_.EnqueueKernels(shape, stream_, timing_ ? stage_ev_ : nullptr);
