@@ -1068,7 +1068,11 @@ private:
             at[0] = root;
             for (size_t i = 1; i < count; ++i) {
                 size_t next = 1;
+#if CUDART_VERSION >= 13000  // (with the edges' data)
+                VQM_CK(cudaGraphNodeGetDependentNodes(at[i - 1], &at[i], nullptr, &next));
+#else
                 VQM_CK(cudaGraphNodeGetDependentNodes(at[i - 1], &at[i], &next));
+#endif
             }
             for (size_t i = 0; i + 1 < count; ++i, ++nodes) {
                 node[i] = at[i];
