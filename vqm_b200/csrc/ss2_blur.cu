@@ -1118,16 +1118,15 @@ cudaError_t LaunchBlur(const DevBatch& b, int variant, cudaStream_t stream) {
     return Dispatch(b, variant, stream, true);
 }
 
-cudaError_t PreloadBlur() {
-    for (int v = 0; v < kBlurVariantCount; ++v)
-        for (int half = 0; half < 2; ++half) {
-            DevBatch b{};
-            b.half = static_cast<uint32_t>(half);
-            const int run = half ? HalfPlaneVariant(v) : v;
-            if (run < 0) continue;
-            const cudaError_t e = Dispatch(b, run, nullptr, false);
-            if (e != cudaSuccess) return e;
-        }
+cudaError_t PreloadBlur(bool half) {
+    DevBatch b{};
+    b.half = half ? 1u : 0u;
+    for (int v = 0; v < kBlurVariantCount; ++v) {
+        const int run = half ? HalfPlaneVariant(v) : v;
+        if (run < 0) continue;
+        const cudaError_t e = Dispatch(b, run, nullptr, false);
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 

@@ -28,10 +28,11 @@ cudaError_t LaunchPrepareOne(const DevBatch& batch, const DevPair& pair,
 // batch's pair_done and seg_done counters must be zero when it starts (the
 // kernel leaves them zero).
 cudaError_t LaunchBlur(const DevBatch& batch, int variant, cudaStream_t stream);
-// Load every kernel of each stage on the current device (and set the blur
-// kernels' shared-memory limits), so that no first launch pays for it.
-cudaError_t PreloadPrepare();
-cudaError_t PreloadBlur();
+// Load every kernel of each stage for float or half planes on the current
+// device (and set the blur kernels' shared-memory limits), so that no first
+// launch pays for it.
+cudaError_t PreloadPrepare(bool half);
+cudaError_t PreloadBlur(bool half);
 // Checks the prepare kernels' cube root against ss2dm::cbrt, bit for bit, on
 // every float whose bit pattern lies in [first_bits, last_bits], on the
 // current device; synchronous.

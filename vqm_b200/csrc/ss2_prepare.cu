@@ -688,9 +688,8 @@ cudaError_t PreloadPrepareOf() {
     if (e == cudaSuccess) e = PreloadPrepareKernels<3, kHalf, 128>();
     return e;
 }
-cudaError_t PreloadPrepare() {
-    const cudaError_t e = PreloadPrepareOf<false>();
-    return e == cudaSuccess ? PreloadPrepareOf<true>() : e;
+cudaError_t PreloadPrepare(bool half) {
+    return half ? PreloadPrepareOf<true>() : PreloadPrepareOf<false>();
 }
 
 namespace {
