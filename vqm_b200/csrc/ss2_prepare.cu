@@ -808,8 +808,8 @@ void LaunchPrepareOf(const Images& images, uint32_t windows420, cudaStream_t str
     if (images.Blocks(2)) images.template Launch<2, kHalf, 256>(stream);
     // The curve decode by the same rule (two waves of its 256-thread CTAs).
     // Against the generic kernel, which these images ran before: 4K ST 2084
-    // 4:2:0 831 -> 415 us a pair, 1080p HLG 4:2:0 151 -> 70, 4000x2667 16-bit
-    // sRGB 628 -> 400, 1001x667 8-bit sRGB with alpha 47 -> 32.
+    // 4:2:0 831 -> 410 us a pair, 1080p HLG 4:2:0 151 -> 69, 3999x2667 16-bit
+    // sRGB 628 -> 398, 1001x667 8-bit sRGB with alpha 47 -> 32.
     if (const uint32_t n = images.Blocks(3)) {
         if ((windows420 & kWindowsCurve) && n >= 2u * 4u * DeviceSmCount())
             images.template Launch<3, kHalf, 128>(stream);
