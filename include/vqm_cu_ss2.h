@@ -325,7 +325,8 @@ typedef struct vqm_cu_ss2_batch_config {
                               from the tile count (a strip length of the
                               default tile; strips regroup the compensated
                               partial sums, so results agree to rounding,
-                              ~1e-7 relative), k = compiled variant k - 1 */
+                              ~1e-7 relative; half planes: the same bits),
+                              k = compiled variant k - 1 */
     uint32_t half_planes;  /* 1: binary16 pyramid planes, as
                               vqm_cu_ss2_config.half_planes */
     uint32_t blur;         /* VQM_CU_SS2_BLUR_*; 0 = VQM's */

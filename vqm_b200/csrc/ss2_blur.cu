@@ -21,7 +21,8 @@
 //      again two lanes per instruction, then evaluates the maps of its eight
 //      pixels and keeps six running sums.
 //   4. The CTA's six sums are combined with two-sum compensation into one
-//      partial per CTA (its tile, or its strip of tiles below).
+//      partial per CTA (its tile, or its strip of tiles below; with half
+//      planes one per tile).
 //   5. The CTA that writes a segment's last partial adds the segment's
 //      partials in FP64, and the one that completes a pair's last segment
 //      turns the pair's sums into its 108 norms and FP64 score (the

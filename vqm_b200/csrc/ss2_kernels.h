@@ -57,7 +57,8 @@ uint32_t BlurBlocks(int index, uint32_t tiles_x, uint32_t tiles_y);
 // segments with these tile grids of the default tile (columns, rows, in
 // launch order) on a device with `sms` SMs: the strip length with the least
 // estimated time (ss2_blur.cu). A strip regroups the compensated partial
-// sums, so the choice moves a result by rounding only (~1e-7 relative).
+// sums, so the choice moves a result by rounding only (~1e-7 relative; with
+// half planes, whose partials are per tile, not at all).
 int AutoBlurVariant(const std::vector<std::pair<uint32_t, uint32_t>>& grids, int sms);
 // The variant half planes run for `variant`: itself, or for a persistent one
 // the one-tile-per-CTA variant of its tile shape; -1 when there is none.

@@ -810,7 +810,8 @@ class Ssimulacra2Batch:
         neither: each submit picks a 32x32 strip length from its tile count
         (strips regroup the compensated partial sums, so results agree to
         rounding, ~1e-7 relative, whichever runs). `half_planes` stores the
-        pyramid as binary16 (ssimulacra2.h:41-46). `blur`: the filter
+        pyramid as binary16 (ssimulacra2.h:41-46); its results are the same
+        bits from every strip length of a tile. `blur`: the filter
         (Ssimulacra2Blur)."""
         tw, th = tile if tile else (0, 0)
         v = 0 if variant is None else variant + 1
